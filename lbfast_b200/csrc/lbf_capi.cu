@@ -89,7 +89,8 @@ void free_all(lbf_handle* h) {
     cudaFree(h->d_err);
     cudaFree(h->d_red);
     cudaFree(h->d_mass);
-    cudaFree(h->bb_nodes);
+    cudaFree(h->wall_nodes);
+    cudaFree(h->wall_links);
     cudaFree(h->d_rnrm);
     cudaFree(h->d_rep);
     cudaFree(h->staging);
@@ -458,25 +459,6 @@ int lbf_set_isfluid(lbf_handle* h, const int8_t* isf) {
     }
     CUDA_TRY(cudaMemcpyAsync(h->isf, isf, h->N, cudaMemcpyHostToDevice, h->stream));
     h->isf_set = true;
-    if (h->p.bounce_back) {
-        // BOUNCE_BACK: the nodes whose wall links the half-way bounce-back rewrites
-        std::vector<long long> nb;
-        const long long plane = (long long)h->nx * h->ny;
-        const long long i_lo = h->slab ? lbf::SLAB_HALO * plane : 0;
-        const long long i_hi = h->slab ? (lbf::SLAB_HALO + h->nzs) * plane : h->N;
-        for (long long i = i_lo; i < i_hi; ++i)
-            if (isf[i] == -1) nb.push_back(i);
-        cudaFree(h->bb_nodes);
-        h->bb_nodes = nullptr;
-        h->nbb = (long long)nb.size();
-        if (h->nbb) {
-            CUDA_TRY(cudaMalloc(&h->bb_nodes, nb.size() * sizeof(long long)));
-            CUDA_TRY(cudaMemcpy(h->bb_nodes, nb.data(), nb.size() * sizeof(long long), cudaMemcpyHostToDevice));
-        }
-    }
-    if (!h->tc) return LBF_OK;
-    // wetting tables: PHI_int_boundary_kernel steps 1-2 (lb_cuda_boundary_module.f90:281-398),
-    // in double; they depend on isfluid only.
     const int pb[3] = {h->p.pbc_x, h->p.pbc_y, h->p.pbc_z};
     const int dims[3] = {nx, ny, nz};
     const int lat = h->p.lattice;
@@ -490,6 +472,44 @@ int lbf_set_isfluid(lbf_handle* h, const int8_t* isf) {
         }
         return isf[((long long)c[2] * ny + c[1]) * nx + c[0]];
     };
+    if (h->p.bounce_back || h->obc_open) {
+        // the nodes whose wall links the passes after the step rewrite, with
+        // those links: BOUNCE_BACK every isfluid = -1 node (of a slab's own
+        // planes), the open faces theirs
+        std::vector<long long> nodes;
+        std::vector<unsigned> links;
+        const int k_lo = h->slab ? lbf::SLAB_HALO : 0, k_hi = h->slab ? lbf::SLAB_HALO + h->nzs : nz;
+        for (int k = k_lo; k < k_hi; ++k)
+            for (int j = 0; j < ny; ++j)
+                for (int i = 0; i < nx; ++i) {
+                    const long long c = ((long long)k * ny + j) * nx + i;
+                    if (isf[c] != -1) continue;
+                    const int at[3] = {i, j, k};
+                    bool take = h->p.bounce_back != 0;
+                    for (int f = 0; f < 6 && !take; ++f) take = lbf::open_face_node(h->obc_open, at, dims, f >> 1, f & 1);
+                    if (!take) continue;
+                    unsigned m = 0;
+                    for (int l = 1; l < 27; ++l)
+                        if (link_in(lat, l) && isf_at(i - EXh[l], j - EYh[l], k - EZh[l]) == 0) m |= 1u << l;
+                    if (!m) continue;  // nothing to rewrite
+                    nodes.push_back(c);
+                    links.push_back(m);
+                }
+        cudaFree(h->wall_nodes);
+        cudaFree(h->wall_links);
+        h->wall_nodes = nullptr;
+        h->wall_links = nullptr;
+        h->nwall = (long long)nodes.size();
+        if (h->nwall) {
+            CUDA_TRY(cudaMalloc(&h->wall_nodes, nodes.size() * sizeof(long long)));
+            CUDA_TRY(cudaMalloc(&h->wall_links, links.size() * sizeof(unsigned)));
+            CUDA_TRY(cudaMemcpy(h->wall_nodes, nodes.data(), nodes.size() * sizeof(long long), cudaMemcpyHostToDevice));
+            CUDA_TRY(cudaMemcpy(h->wall_links, links.data(), links.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+        }
+    }
+    if (!h->tc) return LBF_OK;
+    // wetting tables: PHI_int_boundary_kernel steps 1-2 (lb_cuda_boundary_module.f90:281-398),
+    // in double; they depend on isfluid only.
     std::vector<long long> vs;
     std::vector<int> vd, vf, vsh;
     std::vector<double> vwn;
@@ -1286,16 +1306,22 @@ int handle_post_step(lbf_handle* h) {
     // wall passes on the step's output moments (buffer cur after the advance),
     // from the step's input buffers (1 - cur), which the step left intact:
     // BOUNCE_BACK, then the open faces (bcs_mesoscopic_hfields after the fused kernel)
-    if (h->obc_open || h->nbb) {
+    if (h->nwall) {
         const int in = 1 - h->cur;
         lbf::BoundaryArgs a;
         a.smag = h->p.smagorinsky;
         a.rep = h->d_rep;
-        a.nodes = h->bb_nodes;
-        a.nnodes = h->nbb;
-        a.axis = a.side = a.type = 0;
-        a.press = 0.0;
-        a.vel[0] = a.vel[1] = a.vel[2] = 0.0;
+        a.nodes = h->wall_nodes;
+        a.links = h->wall_links;
+        a.nnodes = h->nwall;
+        a.bounce_back = h->p.bounce_back;
+        a.open = h->obc_open;
+        for (int axis = 0; axis < 3; ++axis)
+            for (int side = 0; side < 2; ++side) {
+                a.type[axis][side] = h->p.openbc_type[axis][side];
+                a.press[axis][side] = h->p.openbc_press[axis][side];
+                for (int d = 0; d < 3; ++d) a.vel[axis][side][d] = h->p.openbc_vel[axis][side][d];
+            }
         a.nx = h->nx; a.ny = h->ny; a.nz = h->nz;
         a.pbx = h->p.pbc_x; a.pby = h->p.pbc_y; a.pbz = h->p.pbc_z;
         a.lattice = h->p.lattice; a.highorder = h->p.highorder; a.tc = h->tc; a.dr = h->dr;
@@ -1309,17 +1335,7 @@ int handle_post_step(lbf_handle* h) {
         a.mom = h->mom[h->cur]; a.pres = h->pres[h->cur];
         for (int f = 0; f < lbf::NSCALE_H; ++f) a.scale[f] = h->scale[f];
         a.mass = h->d_mass;
-        if (h->nbb) CUDA_TRY(lbf::launch_bounce_back(h->storage, a, h->stream));
-        for (int axis = 0; axis < 3; ++axis) {
-            if (!(h->obc_open & (1 << axis))) continue;
-            for (int side = 0; side < 2; ++side) {
-                a.axis = axis; a.side = side;
-                a.type = h->p.openbc_type[axis][side];
-                a.press = h->p.openbc_press[axis][side];
-                for (int d = 0; d < 3; ++d) a.vel[d] = h->p.openbc_vel[axis][side][d];
-                CUDA_TRY(lbf::launch_open_face(h->storage, a, h->stream));
-            }
-        }
+        CUDA_TRY(lbf::launch_walls(h->storage, a, h->stream));
     }
     return LBF_OK;
 }

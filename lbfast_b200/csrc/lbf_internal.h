@@ -138,25 +138,27 @@ enum MassMode { MASS_INITIAL = 0, MASS_SUM = 1, MASS_APPLY = 2 };
 cudaError_t launch_mass(int storage, MassMode mode, long long N, void* phi, const int8_t* isf, double* d_mass,
                         cudaStream_t st);
 
-// Wall passes after a step, on the step's output moments, at isfluid = -1
-// nodes; each recomputes its nodes' moments after the force half-step from the
-// step's input buffers, which the step leaves intact (lbf_walls.cu).
-//  * open face (axis 0/1/2, side 0 low / 1 high): replaces the bounce-back
-//    populations of the wall links by those of the face's state
-//    (boundary_cds_module.f90:57-1311); one launch per face, in the
-//    reference's order x low, x high, y low, ..., z high.
+// Wall passes after a step (lbf_walls.cu), on the step's output moments, at a
+// list of isfluid = -1 nodes; each recomputes its node's moments after the
+// force half-step from the step's input buffers, which the step leaves intact.
 //  * BOUNCE_BACK (lb_cuda_fused_module.f90:20-424): replaces the step's
 //    moment-space bounce-back of the wall links by the half-way bounce-back
-//    of the node's own post-collision populations, over the nodes of `nodes`.
+//    of the node's own post-collision populations.
+//  * open faces: replace the bounce-back populations of the wall links by
+//    those of the face's state (boundary_cds_module.f90:57-1311), at the nodes
+//    of open_face_node, in the reference's order x low, x high, y low, ..., z high.
 struct BoundaryArgs {
     int nx, ny, nz, pbx, pby, pbz;
-    int axis, side, type;       // type: 2 zero gradient, 1 pressure, other velocity
-    double press, vel[3];
+    int bounce_back;            // BOUNCE_BACK at every node of the list
+    int open;                   // open faces: bit 0 x, 1 y, 2 z
+    int type[3][2];             // per axis and side: 2 zero gradient, 1 pressure, other velocity
+    double press[3][2], vel[3][2][3];
     int lattice, highorder, tc, dr;
     double omega, visc1, visc2, rho_r, rho_b, beta, kapp, sharp_c, tau_diff, fx, fy, fz;
     int smag;                   // SMAGORINSKI relaxation in the collision
     const void* rep;            // REPULSIVE_FLUX force of the step (3 x N, arithmetic type), or nullptr
-    const long long* nodes;     // BOUNCE_BACK: the isfluid = -1 nodes
+    const long long* nodes;     // the wall nodes
+    const unsigned* links;      // per wall node: bit l set when the upstream node x - c_l (D3Q27 index) is solid
     long long nnodes;
     const int8_t* isf;
     const void* min;            // the step's input moments
@@ -168,8 +170,15 @@ struct BoundaryArgs {
     double scale[NSCALE_H];
     const double* mass;         // phi mass correction of the step's input phi (see launch_mass), or nullptr
 };
-cudaError_t launch_open_face(int storage, const BoundaryArgs& a, cudaStream_t st);
-cudaError_t launch_bounce_back(int storage, const BoundaryArgs& a, cudaStream_t st);
+// whether a node of a box of n nodes is on the open face (axis, side): on the
+// plane next to the wall, with tangential indices 1 .. n-2
+__host__ __device__ inline bool open_face_node(int open, const int (&c)[3], const int (&n)[3], int axis, int side) {
+    if (!(open >> axis & 1) || c[axis] != (side ? n[axis] - 2 : 1)) return false;
+    for (int d = 0; d < 3; ++d)
+        if (d != axis && (c[d] < 1 || c[d] > n[d] - 2)) return false;
+    return true;
+}
+cudaError_t launch_walls(int storage, const BoundaryArgs& a, cudaStream_t st);
 
 // phi carried through the open faces by a state (BCPHIFLUX,
 // boundary_cds_module.f90:1667-1861): sum over the isfluid = -1 nodes of the

@@ -32,6 +32,8 @@ int grid_for(long long n, int bs) {
     return (int)(b < 1 ? 1 : b);
 }
 
+constexpr int WALL_THREADS = 64;  // a short list still spreads over the SMs
+
 // factor of axis multiplicity m of the D3Q27 Hermite row r in Minv_mrt(r, l)
 // = w_l prod_axes F(m, c): 1, c / cs^2, (c^2 - cs^2) / (2 cs^4)
 __device__ __forceinline__ double hfac(int m, int c) {
@@ -319,31 +321,69 @@ __device__ double collision_omega(const BoundaryArgs& a, const NodeState& ns, co
     return om;
 }
 
-// Open face, one thread per face node; FP64 arithmetic, as the reference's
-// boundary code (real(kind=db)), on every storage type.
+// The wall passes of a step, one thread per wall node of the list: BOUNCE_BACK,
+// then the open faces of the node in the reference's order (x low, x high,
+// y low, ...; a node at an edge of the box has several).  FP64 arithmetic, as
+// the reference's boundary code (real(kind=db)), on every storage type.  A
+// node's passes read only its own moments and force (node_state) and its wall
+// links, so one launch does them all and the moments stay in registers
+// between them.
+//
+// BOUNCE_BACK: the step added for each wall link l (upstream x - c_l solid)
+// the moment-space population w_l P + (1 - omega) fneq (LB_int_boundary,
+// lb_cuda_boundary_module.f90:162-199) and the solid node's push, which is
+// zero; fused_LB_kernel_bb (lb_cuda_fused_module.f90:364-380) brings instead
+// the node's own post-collision population of the opposite link
+// (lb_cuda_fused_module.f90:637-713).  P and fneq are even in c, so the two
+// differ by the odd and higher terms only, which are added here.
+//
+// Bound by the latency of a node's FP64 chain: the list is a few per cent of
+// the box.  The solid tests are a bit mask per node, made with the list; they
+// were 26 loads of isfluid with a wrapped index each.  160 x 96 x 80 D3Q19
+// with two open axes and 24 spheres (BOUNCE_BACK and four faces): the step
+// and its wall passes 189 us as five launches, 135 us as one.
 template <typename S, int LAT, bool HO>
-__global__ void open_face_kernel(const BoundaryArgs a) {
-    const int n[3] = {a.nx, a.ny, a.nz};
-    const int a1 = a.axis == 0 ? 1 : 0, a2 = a.axis == 2 ? 1 : 2;
-    const int m1 = n[a1] - 2, m2 = n[a2] - 2;
-    if (m1 <= 0 || m2 <= 0) return;
-    const long long tot = (long long)m1 * m2;
+__global__ void __launch_bounds__(WALL_THREADS) wall_kernel(const BoundaryArgs a) {
     const long long plane = (long long)a.nx * a.ny, N = plane * a.nz;
     const double cssq = 1.0 / 3.0;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
-         t += (long long)gridDim.x * blockDim.x) {
-        int x[3];
-        x[a.axis] = a.side ? n[a.axis] - 2 : 1;
-        x[a1] = 1 + (int)(t % m1);
-        x[a2] = 1 + (int)(t / m1);
-        const long long g = x[2] * plane + (long long)x[1] * a.nx + x[0];
-        if (a.isf[g] != -1) continue;
-        NodeState ns;
-        node_state<S>(a, x[0], x[1], x[2], g, ns);
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= a.nnodes) return;
+    const long long g = a.nodes[t];
+    const unsigned links = a.links[t];
+    const int z = (int)(g / plane), y = (int)((g - z * plane) / a.nx), x = (int)(g - z * plane - (long long)y * a.nx);
+    NodeState ns;
+    node_state<S>(a, x, y, z, g, ns);
+    const double P = ns.m[0], u = ns.m[1], v = ns.m[2], w = ns.m[3];
+    const double inv = a.dr ? 1.0 / ns.rhophi : 1.0;
+    double o[10];
+    load_out<S>(a, g, N, o);
+    if (a.bounce_back) {
+        const double pn[6] = {ns.m[4] - u * u, ns.m[5] - v * v, ns.m[6] - w * w,
+                              ns.m[7] - u * v, ns.m[8] - u * w, ns.m[9] - v * w};
+        const double om = collision_omega(a, ns, pn);
+        const double Fx = ns.tf[0] * inv, Fy = ns.tf[1] * inv, Fz = ns.tf[2] * inv;
+        const double uu = 0.5 * (u * u + v * v + w * w) * 3.0;
+        double hm[17];
+        if constexpr (HO) ho_coeffs(u, v, w, pn, 1.0 - om, hm);
+#pragma unroll
+        for (int l = 1; l < 27; ++l) {
+            if (!IN<LAT>(l) || !(links >> l & 1)) continue;
+            // the opposite link's population, arriving as link l
+            const double wl = WL<LAT>(l);
+            const double dx = EX(l), dy = EY(l), dz = EZ(l);
+            const double ex = -dx, ey = -dy, ez = -dz;
+            const double ud = (u * ex + v * ey + w * ez) * 3.0;
+            double f = ud + 0.5 * ud * ud - uu;
+            if constexpr (HO) f += ho_sum(-EX(l), -EY(l), -EZ(l), hm);
+            f += 1.5 * (((ex - u) + ud * ex) * Fx + ((ey - v) + ud * ey) * Fy + ((ez - w) + ud * ez) * Fz);
+            add_link(o, wl * f, dx, dy, dz);
+        }
+    }
+    if (a.open) {
+        const int c[3] = {x, y, z}, n[3] = {a.nx, a.ny, a.nz};
         // Pi' = Pi - cs^2 P - u u of the node's moments after the force half-step
-        const double press = ns.m[0], u = ns.m[1], v = ns.m[2], w = ns.m[3];
-        const double pq[6] = {ns.m[4] - cssq * press - u * u, ns.m[5] - cssq * press - v * v,
-                              ns.m[6] - cssq * press - w * w, ns.m[7] - u * v, ns.m[8] - u * w, ns.m[9] - v * w};
+        const double pq[6] = {ns.m[4] - cssq * P - u * u, ns.m[5] - cssq * P - v * v, ns.m[6] - cssq * P - w * w,
+                              ns.m[7] - u * v, ns.m[8] - u * w, ns.m[9] - v * w};
         // the molecular relaxation rate (boundary_cds_module.f90:151-162)
         double om = a.omega;
         if (a.tc) {
@@ -351,95 +391,41 @@ __global__ void open_face_kernel(const BoundaryArgs a) {
             om = 1.0 / (visc * 3.0 + 0.5);
         }
         const double om1 = 1.0 - om;
-        double pb = press, ub = u, vb = v, wb = w;
-        if (a.type == 1) {
-            pb = a.press;
-        } else if (a.type != 2) {
-            ub = a.vel[0]; vb = a.vel[1]; wb = a.vel[2];
-        }
-        const double uu = 0.5 * (ub * ub + vb * vb + wb * wb) * 3.0;
-        double hm[17];
-        if constexpr (HO) ho_coeffs(ub, vb, wb, pq, om1, hm);
-        double o[10];
-        load_out<S>(a, g, N, o);
+#pragma unroll 1
+        for (int face = 0; face < 6; ++face) {
+            const int axis = face >> 1, side = face & 1;
+            if (!open_face_node(a.open, c, n, axis, side)) continue;
+            const int type = a.type[axis][side];
+            double pb = P, ub = u, vb = v, wb = w;
+            if (type == 1) {
+                pb = a.press[axis][side];
+            } else if (type != 2) {
+                ub = a.vel[axis][side][0]; vb = a.vel[axis][side][1]; wb = a.vel[axis][side][2];
+            }
+            const double uu = 0.5 * (ub * ub + vb * vb + wb * wb) * 3.0;
+            double hm[17];
+            if constexpr (HO) ho_coeffs(ub, vb, wb, pq, om1, hm);
 #pragma unroll
-        for (int l = 1; l < 27; ++l) {
-            if (!IN<LAT>(l)) continue;
-            const int cx = EX(l), cy = EY(l), cz = EZ(l);
-            // upstream node x - c_l: inside the box (the face nodes keep one
-            // node away from every box face)
-            const long long gu = g - ((long long)cz * plane + (long long)cy * a.nx + cx);
-            if (a.isf[gu] != 0) continue;
-            const double wl = WL<LAT>(l);
-            const double dx = cx, dy = cy, dz = cz;
-            const double qn = qform(dx, dy, dz, pq);
-            // the bounce-back population, taken out with the weights c_a c_b
-            const double fo = wl * press + om1 * (wl * qn);
-            o[0] -= fo;
-            o[1] -= fo * dx; o[2] -= fo * dy; o[3] -= fo * dz;
-            o[4] -= fo * (dx * dx); o[5] -= fo * (dy * dy); o[6] -= fo * (dz * dz);
-            o[7] -= fo * (dx * dy); o[8] -= fo * (dx * dz); o[9] -= fo * (dy * dz);
-            // the face's population
-            const double udotc = (ub * dx + vb * dy + wb * dz) * 3.0;
-            double fn = wl * (pb + udotc + 0.5 * udotc * udotc - uu) + om1 * (wl * qn);
-            if constexpr (HO) fn += wl * ho_sum(cx, cy, cz, hm);
-            add_link(o, fn, dx, dy, dz);
+            for (int l = 1; l < 27; ++l) {
+                if (!IN<LAT>(l) || !(links >> l & 1)) continue;
+                const double wl = WL<LAT>(l);
+                const double dx = EX(l), dy = EY(l), dz = EZ(l);
+                const double qn = om1 * (wl * qform(dx, dy, dz, pq));
+                // the bounce-back population, taken out with the weights c_a c_b
+                const double fo = wl * P + qn;
+                o[0] -= fo;
+                o[1] -= fo * dx; o[2] -= fo * dy; o[3] -= fo * dz;
+                o[4] -= fo * (dx * dx); o[5] -= fo * (dy * dy); o[6] -= fo * (dz * dz);
+                o[7] -= fo * (dx * dy); o[8] -= fo * (dx * dz); o[9] -= fo * (dy * dz);
+                // the face's population
+                const double udotc = (ub * dx + vb * dy + wb * dz) * 3.0;
+                double fn = wl * (pb + udotc + 0.5 * udotc * udotc - uu) + qn;
+                if constexpr (HO) fn += wl * ho_sum(EX(l), EY(l), EZ(l), hm);
+                add_link(o, fn, dx, dy, dz);
+            }
         }
-        store_out<S>(a, g, N, o);
     }
-}
-
-// BOUNCE_BACK, one thread per isfluid = -1 node.  The step added for each
-// wall link l (upstream x - c_l solid) the moment-space population
-// w_l P + (1 - omega) fneq (LB_int_boundary, lb_cuda_boundary_module.f90:162-199)
-// and the solid node's push, which is zero; fused_LB_kernel_bb
-// (lb_cuda_fused_module.f90:364-380) brings instead the node's own
-// post-collision population of the opposite link.  FP64.
-template <typename S, int LAT, bool HO>
-__global__ void bounce_back_kernel(const BoundaryArgs a) {
-    const long long plane = (long long)a.nx * a.ny, N = plane * a.nz;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < a.nnodes;
-         t += (long long)gridDim.x * blockDim.x) {
-        const long long g = a.nodes[t];
-        const int z = (int)(g / plane), y = (int)((g - z * plane) / a.nx), x = (int)(g - z * plane - (long long)y * a.nx);
-        NodeState ns;
-        node_state<S>(a, x, y, z, g, ns);
-        const double P = ns.m[0], u = ns.m[1], v = ns.m[2], w = ns.m[3];
-        const double pn[6] = {ns.m[4] - u * u, ns.m[5] - v * v, ns.m[6] - w * w,
-                              ns.m[7] - u * v, ns.m[8] - u * w, ns.m[9] - v * w};
-        const double om = collision_omega(a, ns, pn);
-        const double om1 = 1.0 - om;
-        const double inv = a.dr ? 1.0 / ns.rhophi : 1.0;
-        const double Fx = ns.tf[0] * inv, Fy = ns.tf[1] * inv, Fz = ns.tf[2] * inv;
-        const double uu = 0.5 * (u * u + v * v + w * w) * 3.0;
-        double hm[17];
-        if constexpr (HO) ho_coeffs(u, v, w, pn, om1, hm);
-        double o[10];
-        load_out<S>(a, g, N, o);
-#pragma unroll
-        for (int l = 1; l < 27; ++l) {
-            if (!IN<LAT>(l)) continue;
-            const int cx = EX(l), cy = EY(l), cz = EZ(l);
-            bool ok = true;
-            const int ux = wrap_coord(x - cx, a.nx, a.pbx, ok), uy = wrap_coord(y - cy, a.ny, a.pby, ok);
-            const int uz = wrap_coord(z - cz, a.nz, a.pbz, ok);
-            if (!ok || a.isf[(long long)uz * plane + (long long)uy * a.nx + ux] != 0) continue;
-            const double dx = cx, dy = cy, dz = cz;
-            // out: the moment-space population of link l the step added
-            const double wl = WL<LAT>(l);
-            add_link(o, -(wl * P + om1 * (wl * qform(dx, dy, dz, pn))), dx, dy, dz);
-            // in: the node's post-collision population of the opposite link,
-            // arriving as link l (lb_cuda_fused_module.f90:637-713)
-            const double ex = -dx, ey = -dy, ez = -dz;
-            const double ud = (u * ex + v * ey + w * ez) * 3.0;
-            double feq = wl * (P + ud + 0.5 * ud * ud - uu);
-            double fne = om1 * (wl * qform(ex, ey, ez, pn));
-            if constexpr (HO) feq += wl * ho_sum(-cx, -cy, -cz, hm);
-            const double fd = wl * (((ex - u) + ud * ex) * Fx + ((ey - v) + ud * ey) * Fy + ((ez - w) + ud * ez) * Fz) * 3.0;
-            add_link(o, feq + fne + 0.5 * fd, dx, dy, dz);
-        }
-        store_out<S>(a, g, N, o);
-    }
+    store_out<S>(a, g, N, o);
 }
 
 template <typename S>
@@ -479,30 +465,15 @@ __global__ void phi_flux_kernel(int nx, int ny, int nz, int axis, int side, cons
 
 }  // namespace
 
-cudaError_t launch_open_face(int storage, const BoundaryArgs& a, cudaStream_t st) {
-    const int n[3] = {a.nx, a.ny, a.nz};
-    const long long tot = (long long)(n[a.axis == 0 ? 1 : 0] - 2) * (n[a.axis == 2 ? 1 : 2] - 2);
-    if (tot <= 0 || n[a.axis] < 3) return cudaSuccess;
-    const int grid = grid_for(tot, 128);
-    return by_storage(storage, [&](auto tag) {
-        using S = decltype(tag);
-        if (a.lattice == 27 && a.highorder) open_face_kernel<S, 27, true><<<grid, 128, 0, st>>>(a);
-        else if (a.lattice == 27) open_face_kernel<S, 27, false><<<grid, 128, 0, st>>>(a);
-        else if (a.lattice == 19) open_face_kernel<S, 19, false><<<grid, 128, 0, st>>>(a);
-        else open_face_kernel<S, 15, false><<<grid, 128, 0, st>>>(a);
-        return cudaGetLastError();
-    });
-}
-
-cudaError_t launch_bounce_back(int storage, const BoundaryArgs& a, cudaStream_t st) {
+cudaError_t launch_walls(int storage, const BoundaryArgs& a, cudaStream_t st) {
     if (a.nnodes <= 0) return cudaSuccess;
-    const int grid = grid_for(a.nnodes, 128);
+    const unsigned grid = (unsigned)((a.nnodes + WALL_THREADS - 1) / WALL_THREADS);
     return by_storage(storage, [&](auto tag) {
         using S = decltype(tag);
-        if (a.lattice == 27 && a.highorder) bounce_back_kernel<S, 27, true><<<grid, 128, 0, st>>>(a);
-        else if (a.lattice == 27) bounce_back_kernel<S, 27, false><<<grid, 128, 0, st>>>(a);
-        else if (a.lattice == 19) bounce_back_kernel<S, 19, false><<<grid, 128, 0, st>>>(a);
-        else bounce_back_kernel<S, 15, false><<<grid, 128, 0, st>>>(a);
+        if (a.lattice == 27 && a.highorder) wall_kernel<S, 27, true><<<grid, WALL_THREADS, 0, st>>>(a);
+        else if (a.lattice == 27) wall_kernel<S, 27, false><<<grid, WALL_THREADS, 0, st>>>(a);
+        else if (a.lattice == 19) wall_kernel<S, 19, false><<<grid, WALL_THREADS, 0, st>>>(a);
+        else wall_kernel<S, 15, false><<<grid, WALL_THREADS, 0, st>>>(a);
         return cudaGetLastError();
     });
 }

@@ -43,3 +43,21 @@ def test_film_search(box, pbc, q_th, cos):
     phi = _blobs(rng, p.shape, 6, 2.0, 4.0, 2.5)
     m = _random_moments(rng, p.shape, amp_u=0.002, amp_p=0.0005, amp_neq=1e-6)
     _compare(p, np.ones(p.shape, np.int8), m, phi, 3)
+
+
+@pytest.mark.parametrize("box,pbc,bb,types", [
+    ((3, 12, 9), (0, 1, 1), 0, ((1, 1), (0, 0), (0, 0))), ((3, 3, 14), (0, 0, 1), 1, ((0, 0), (1, 2), (0, 0))),
+    ((20, 11, 3), (1, 1, 0), 1, ((0, 0), (0, 0), (0, 0))), ((33, 9, 8), (0, 0, 0), 1, ((1, 2), (0, 0), (0, 0)))])
+@pytest.mark.parametrize("lattice,highorder", [(15, 0), (19, 0), (27, 1)])
+def test_wall_passes(box, pbc, bb, types, lattice, highorder):
+    lx, ly, lz = box
+    rng = np.random.default_rng(lx * 100 + lz)
+    p = Params(lx=lx, ly=ly, lz=lz, pbc_x=pbc[0], pbc_y=pbc[1], pbc_z=pbc[2], lattice=lattice, highorder=highorder,
+               obstacles=1, bounce_back=bb, visc1=0.1, storage="f64", openbc=1, openbc_type=types,
+               openbc_press=((0.002, -0.002),) * 3, fx=1e-6)
+    solid = np.zeros(p.shape, dtype=bool)
+    if min(box) > 3:
+        solid[3:5, 3:6, 10:14] = True
+    isf = O.mark_isfluid(solid, pbc, lattice, True)
+    m = np.where((isf == 0)[None], 0.0, _random_moments(rng, p.shape, amp_u=0.003, amp_p=0.002))
+    _compare(p, isf, m, None, 4)
