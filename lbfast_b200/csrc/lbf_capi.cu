@@ -72,6 +72,16 @@ int ensure_staging(lbf_handle* h, size_t bytes) {
     return LBF_OK;
 }
 
+// a device table with the values of v in the place of t
+template <typename T> int replace_table(T*& t, const std::vector<T>& v) {
+    cudaFree(t);
+    t = nullptr;
+    if (v.empty()) return LBF_OK;
+    CUDA_TRY(cudaMalloc(&t, v.size() * sizeof(T)));
+    CUDA_TRY(cudaMemcpy(t, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    return LBF_OK;
+}
+
 void free_all(lbf_handle* h) {
     for (int b = 0; b < 2; ++b) {
         cudaFree(h->mom[b]);
@@ -81,6 +91,8 @@ void free_all(lbf_handle* h) {
         cudaFree(h->wetW[b]);
     }
     cudaFree(h->isf);
+    cudaFree(h->link_rows);
+    cudaFree(h->links);
     cudaFree(h->wet_s);
     cudaFree(h->wet_donor);
     cudaFree(h->wet_flag);
@@ -488,40 +500,50 @@ int lbf_set_isfluid(lbf_handle* h, const int8_t* isf) {
         }
         return isf[((long long)c[2] * ny + c[1]) * nx + c[0]];
     };
-    if (h->p.bounce_back || h->obc_open) {
-        // the nodes whose wall links the passes after the step rewrite, with
-        // those links: BOUNCE_BACK every isfluid = -1 node (of a slab's own
-        // planes), the open faces theirs
-        std::vector<long long> nodes;
-        std::vector<unsigned> links;
+    // wall links of every isfluid = -1 node (bit l: the upstream node x - c_l is
+    // solid), row by row in the step kernel's 32-wide x segments; and the nodes
+    // whose links the passes after the step rewrite: BOUNCE_BACK every -1 node
+    // (of a slab's own planes), the open faces theirs
+    {
+        const int segs = (nx + lbf::STEP_TILE_X - 1) / lbf::STEP_TILE_X;
         const int k_lo = h->slab ? lbf::SLAB_HALO : 0, k_hi = h->slab ? lbf::SLAB_HALO + h->nzs : nz;
-        for (int k = k_lo; k < k_hi; ++k)
-            for (int j = 0; j < ny; ++j)
+        const bool passes = h->p.bounce_back || h->obc_open;
+        std::vector<int> rows((size_t)nz * ny * segs);
+        std::vector<unsigned> links, wall_links;
+        std::vector<long long> wall_nodes;
+        long long up[27];
+        for (int l = 0; l < 27; ++l) up[l] = -(((long long)EZh[l] * ny + EYh[l]) * nx + EXh[l]);
+        for (int k = 0; k < nz; ++k)
+            for (int j = 0; j < ny; ++j) {
+                const int8_t* row = isf + ((long long)k * ny + j) * nx;
+                const bool edge = k == 0 || k == nz - 1 || j == 0 || j == ny - 1;
                 for (int i = 0; i < nx; ++i) {
-                    const long long c = ((long long)k * ny + j) * nx + i;
-                    if (isf[c] != -1) continue;
+                    if (i % lbf::STEP_TILE_X == 0)
+                        rows[((size_t)k * ny + j) * segs + i / lbf::STEP_TILE_X] = (int)links.size();
+                    if (row[i] != -1) continue;
+                    unsigned m = 0;
+                    for (int l = 1; l < 27; ++l) {
+                        if (!link_in(lat, l)) continue;
+                        const int f = edge || i == 0 || i == nx - 1 ? isf_at(i - EXh[l], j - EYh[l], k - EZh[l])
+                                                                    : row[i + up[l]];
+                        if (f == 0) m |= 1u << l;
+                    }
+                    links.push_back(m);
+                    if (!passes || !m || k < k_lo || k >= k_hi) continue;
                     const int at[3] = {i, j, k};
                     bool take = h->p.bounce_back != 0;
                     for (int f = 0; f < 6 && !take; ++f) take = lbf::open_face_node(h->obc_open, at, dims, f >> 1, f & 1);
                     if (!take) continue;
-                    unsigned m = 0;
-                    for (int l = 1; l < 27; ++l)
-                        if (link_in(lat, l) && isf_at(i - EXh[l], j - EYh[l], k - EZh[l]) == 0) m |= 1u << l;
-                    if (!m) continue;  // nothing to rewrite
-                    nodes.push_back(c);
-                    links.push_back(m);
+                    wall_nodes.push_back(row - isf + i);
+                    wall_links.push_back(m);
                 }
-        cudaFree(h->wall_nodes);
-        cudaFree(h->wall_links);
-        h->wall_nodes = nullptr;
-        h->wall_links = nullptr;
-        h->nwall = (long long)nodes.size();
-        if (h->nwall) {
-            CUDA_TRY(cudaMalloc(&h->wall_nodes, nodes.size() * sizeof(long long)));
-            CUDA_TRY(cudaMalloc(&h->wall_links, links.size() * sizeof(unsigned)));
-            CUDA_TRY(cudaMemcpy(h->wall_nodes, nodes.data(), nodes.size() * sizeof(long long), cudaMemcpyHostToDevice));
-            CUDA_TRY(cudaMemcpy(h->wall_links, links.data(), links.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
-        }
+            }
+        int rc = replace_table(h->link_rows, rows);
+        if (!rc) rc = replace_table(h->links, links);
+        if (!rc) rc = replace_table(h->wall_nodes, wall_nodes);
+        if (!rc) rc = replace_table(h->wall_links, wall_links);
+        if (rc) return rc;
+        h->nwall = (long long)wall_nodes.size();
     }
     if (!h->tc) return LBF_OK;
     // wetting tables: PHI_int_boundary_kernel steps 1-2 (lb_cuda_boundary_module.f90:281-398),
@@ -1257,6 +1279,8 @@ void handle_step_args(const lbf_handle* h, StepArgs& a, bool write_u) {
     a.fx = h->p.fx; a.fy = h->p.fy; a.fz = h->p.fz;
     for (int i = 0; i < NSCALE_H; ++i) a.scale[i] = h->scale[i];
     a.isf = h->obs ? h->isf : nullptr;
+    a.link_rows = h->link_rows;
+    a.links = h->links;
     a.err = h->d_err;
     a.rep = h->d_rep;
     a.mass = h->d_mass;

@@ -22,6 +22,8 @@ struct lbf_handle {
     float* pres[2] = {nullptr, nullptr};  // P in FP32 when the other moments are 16-bit
     int8_t* isf = nullptr;
     bool isf_set = false;
+    int* link_rows = nullptr;    // wall links of the isfluid = -1 nodes, by rows (see StepParams)
+    unsigned* links = nullptr;
     int cur = 0;
     long long step = 0;
     bool fields_set = false, primed = false;

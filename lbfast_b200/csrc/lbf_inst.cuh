@@ -38,6 +38,8 @@ template <typename S, typename R> void make_params(const StepArgs& a, StepParams
     p.pres_in = a.pres_in;
     p.pres_out = a.pres_out;
     p.isf = a.isf;
+    p.link_rows = a.link_rows;
+    p.links = a.links;
     p.err = a.err;
     p.rep = static_cast<const R*>(a.rep);
     p.mass = a.mass;
@@ -46,7 +48,7 @@ template <typename S, typename R> void make_params(const StepArgs& a, StepParams
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
 cudaError_t launch_stream(const StepArgs& a, cudaStream_t st) {
     static bool attr_set = false;
-    const size_t smem = stream_smem_bytes<LAT, TC, S, R, TYV>();
+    const size_t smem = step_smem_bytes<LAT, TC, S, R, TYV>();
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -60,24 +62,24 @@ cudaError_t launch_stream(const StepArgs& a, cudaStream_t st) {
     if (a.zseg < 0) {
         // split columns: a head and a tail segment per column
         const long long ncols = (long long)((a.nx + TX - 1) / TX) * ((a.ny + TYV - 1) / TYV);
-        stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<(unsigned)(2 * ncols), TX * TYV, smem, st>>>(p);
+        stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<(unsigned)(2 * ncols), step_threads<TC, TYV>(), smem, st>>>(p);
         return cudaGetLastError();
     }
     if (a.zseg > 0) {
         dim3 grid((a.nx + TX - 1) / TX, (a.ny + TYV - 1) / TYV, (nzr + a.zseg - 1) / a.zseg);
-        stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<grid, TX * TYV, smem, st>>>(p);
+        stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<grid, step_threads<TC, TYV>(), smem, st>>>(p);
         return cudaGetLastError();
     }
     static int resident = 0;  // CTAs per SM at this shared-memory size
     if (!resident) {
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS>,
-                                                                      TX * TYV, smem);
+                                                                      step_threads<TC, TYV>(), smem);
         if (e != cudaSuccess) return e;
         if (resident < 1) return cudaErrorInvalidConfiguration;
     }
     const long long W = (long long)((a.nx + TX - 1) / TX) * ((a.ny + TYV - 1) / TYV) * nzr;
     const int grid = persistent_grid(W, resident);
-    stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<grid, TX * TYV, smem, st>>>(p);
+    stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<grid, step_threads<TC, TYV>(), smem, st>>>(p);
     return cudaGetLastError();
 }
 
@@ -87,7 +89,7 @@ cudaError_t launch_stream(const StepArgs& a, cudaStream_t st) {
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
 cudaError_t launch_stream_batched(const void* d_boxes, const int4* d_work, int nwork, cudaStream_t st) {
     static bool attr_set = false;
-    const size_t smem = stream_smem_bytes<LAT, TC, S, R, TYV>();
+    const size_t smem = step_smem_bytes<LAT, TC, S, R, TYV>();
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(stream_kernel_batched<LAT, HO, TC, S, R, TYV, REP, OBS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -96,18 +98,18 @@ cudaError_t launch_stream_batched(const void* d_boxes, const int4* d_work, int n
     }
     if (nwork <= 0) return cudaSuccess;
     stream_kernel_batched<LAT, HO, TC, S, R, TYV, REP, OBS>
-        <<<nwork, TX * TYV, smem, st>>>(static_cast<const StepParams<S, R>*>(d_boxes), d_work);
+        <<<nwork, step_threads<TC, TYV>(), smem, st>>>(static_cast<const StepParams<S, R>*>(d_boxes), d_work);
     return cudaGetLastError();
 }
 
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true> int batched_resident() {
     static int resident = 0;
     if (!resident) {
-        const size_t smem = stream_smem_bytes<LAT, TC, S, R, TYV>();
+        const size_t smem = step_smem_bytes<LAT, TC, S, R, TYV>();
         if (cudaFuncSetAttribute(stream_kernel_batched<LAT, HO, TC, S, R, TYV, REP, OBS>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, stream_kernel_batched<LAT, HO, TC, S, R, TYV, REP, OBS>,
-                                                          TX * TYV, smem) != cudaSuccess)
+                                                          step_threads<TC, TYV>(), smem) != cudaSuccess)
             resident = 1;
         resident = std::max(resident, 1);
     }

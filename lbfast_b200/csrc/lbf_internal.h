@@ -26,6 +26,8 @@ struct StepArgs {
     const float* pres_in;   // P, u, v, w with 16-bit storage (4 x N)
     float* pres_out;
     const int8_t* isf;
+    const int* link_rows;       // wall links of the isfluid = -1 nodes (see StepParams), or nullptr
+    const unsigned* links;
     int* err;
     const void* rep;        // REPULSIVE_FLUX force of the step (3 x N, arithmetic type), or nullptr
     const double* mass;     // phi mass correction: sums of the step's input phi (see launch_mass), or nullptr

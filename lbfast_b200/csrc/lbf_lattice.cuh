@@ -192,6 +192,8 @@ template <typename S, typename R> struct StepParams {
     const typename PhiStore<S>::type* pin;  // N phase field, input
     typename PhiStore<S>::type* pout;       // N phase field, output (fluid nodes)
     const int8_t* isf;  // N isfluid (obstacles), else nullptr
+    const int* link_rows;   // per (z, y, 32-wide x segment): first entry of its isfluid = -1 nodes in links
+    const unsigned* links;  // per isfluid = -1 node: bit l set when the upstream node x - c_l is solid
     int* err;         // device error word
     const R* rep;     // REPULSIVE_FLUX force (3 x N), else nullptr
     const double* mass;  // phi mass correction of the input phi (see mass_corr), else nullptr

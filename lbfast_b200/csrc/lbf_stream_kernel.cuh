@@ -13,47 +13,10 @@
 //            pulls the populations of plane q and plane q-1 is written.  The
 //            copy completes behind this phase.
 #pragma once
-#include "lbf_stream.cuh"
+#include "lbf_node.cuh"
+#include "lbf_single_kernel.cuh"
 
 namespace lbf {
-
-// Reciprocal and square root: in FP32 the hardware approximations (about 2 ulp)
-// instead of the correctly rounded sequences, which cost several instructions
-// and a branch each; FP64 stays correctly rounded.
-template <typename R> __device__ __forceinline__ R rcp(R x);
-template <> __device__ __forceinline__ float rcp<float>(float x) { return __fdividef(1.0f, x); }
-template <> __device__ __forceinline__ double rcp<double>(double x) { return 1.0 / x; }
-template <typename R> __device__ __forceinline__ R sqrt_a(R x);
-template <> __device__ __forceinline__ float sqrt_a<float>(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
-template <> __device__ __forceinline__ double sqrt_a<double>(double x) { return sqrt(x); }
-
-template <typename R>
-__device__ __forceinline__ void accum_slice(R (&acc)[10], R cz, R Y00, R Y01, R Y02, R Y10, R Y11, R Y20) {
-    acc[0] += Y00;
-    acc[1] += Y10;
-    acc[2] += Y01;
-    acc[3] += cz * Y00;
-    acc[4] += Y20;
-    acc[5] += Y02;
-    acc[6] += (cz * cz) * Y00;
-    acc[7] += Y11;
-    acc[8] += cz * Y10;
-    acc[9] += cz * Y01;
-}
-
-// asynchronous global -> shared copies of 4 or 8 bytes
-template <int BYTES> __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    if constexpr (BYTES == 4) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-    } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-    }
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// Smagorinsky constant of the reference: the single-precision product 0.053 * 18.0
-constexpr double SMAG_C = (double)(0.053f * 18.0f);
 
 // The moments (and u_old) of a collision node go from global memory straight
 // into registers: the tile-interior node's one plane ahead (NodeRaw, below),
@@ -67,55 +30,21 @@ constexpr double SMAG_C = (double)(0.053f * 18.0f);
 // ring slots of the separable phase-field stencils (see step_body)
 constexpr int SXY_SLOTS = 5, GXY_SLOTS = 3, TH_SLOTS = 2, GT_SLOTS = 3, H_SLOTS = 3;
 
-// vector of two R (the populations of cz = -1 and 0 of one (cx, cy) group)
-template <typename R> struct Vec2;
-template <> struct Vec2<float> { using type = float2; };
-template <> struct Vec2<double> { using type = double2; };
-
-// Pairs of independent values in one instruction: FP32 as f32x2 (FFMA2,
-// FADD2, FMUL2 of sm_100: two lanes' operations per issue slot, each rounded
-// as the scalar instruction), FP64 as two scalar operations
-template <typename R> struct PK;
-template <> struct PK<float> {
-    using T = float2;
-    static __device__ __forceinline__ float2 mk(float a, float b) { return make_float2(a, b); }
-    static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-    static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-    static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-};
-template <> struct PK<double> {
-    using T = double2;
-    static __device__ __forceinline__ double2 mk(double a, double b) { return make_double2(a, b); }
-    static __device__ __forceinline__ double2 fma(double2 a, double2 b, double2 c) {
-        return make_double2(::fma(a.x, b.x, c.x), ::fma(a.y, b.y, c.y));
+// asynchronous global -> shared copies of 4 or 8 bytes
+template <int BYTES> __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    if constexpr (BYTES == 4) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+    } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
     }
-    static __device__ __forceinline__ double2 add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-    static __device__ __forceinline__ double2 mul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
-};
-// d1q3_inv with the second coefficient negated (m2n = -m2), the same
-// roundings: scalar and packed
-template <typename R> __device__ __forceinline__ void d1q3n(R m0, R m1, R m2n, R& vm, R& v0, R& vp) {
-    const R s = fmaf_t(m0, R(1.0 / 6.0), R(-0.5) * m2n);
-    const R d = R(0.5) * m1;
-    vm = s - d;
-    vp = s + d;
-    v0 = fmaf_t(m0, R(2.0 / 3.0), m2n);
 }
-template <typename R, typename T = typename PK<R>::T>
-__device__ __forceinline__ void d1q3n2(T m0, T m1, T m2n, T& vm, T& v0, T& vp) {
-    using P = PK<R>;
-    const T s = P::fma(m0, P::mk(R(1.0 / 6.0), R(1.0 / 6.0)), P::mul(P::mk(R(-0.5), R(-0.5)), m2n));
-    const T d = P::mul(P::mk(R(0.5), R(0.5)), m1);
-    vm = P::fma(d, P::mk(R(-1), R(-1)), s);
-    vp = P::add(s, d);
-    v0 = P::fma(m0, P::mk(R(2.0 / 3.0), R(2.0 / 3.0)), m2n);
-}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-template <int LAT, bool TC, typename S, typename R, int TYV> constexpr size_t stream_smem_bytes() {
+template <typename S, typename R, int TYV> constexpr size_t stream_smem_bytes() {
     constexpr int R1N = Tile<TYV>::R1N, R2N = Tile<TYV>::R2N, R3N = Tile<TYV>::R3N;
     size_t b = sizeof(R) * size_t(24) * R1N;  // populations: 8 (cx, cy) groups x 3 cz (the centre stays in registers)
-    if (TC)
-        b += sizeof(R) * (size_t(PHI_SLOTS) * R3N + size_t(SXY_SLOTS) * R2N + size_t(GXY_SLOTS) * 2 * R2N +
+    b += sizeof(R) * (size_t(PHI_SLOTS) * R3N + size_t(SXY_SLOTS) * R2N + size_t(GXY_SLOTS) * 2 * R2N +
                           size_t(TH_SLOTS) * 3 * R2N + size_t(GT_SLOTS) * 3 * R1N + size_t(H_SLOTS) * 3 * R1N);
     return b;
 }
@@ -125,7 +54,7 @@ template <int LAT, bool TC, typename S, typename R, int TYV> constexpr size_t st
 // tests, the moment-space bounce-back, open-face moments).  Both are separate
 // compilations, so the kernels without them carry no code for them: the
 // obstacle code alone, never executed, costs a box without obstacles 5.6 %.
-template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
+template <int LAT, bool HO, typename S, typename R, int TYV, bool REP, bool OBS>
 __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int bx, const int by, const int z0,
                                           const int z1) {
     using TL = Tile<TYV>;
@@ -142,13 +71,20 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     // output, the thread that collided it: it stays in registers)
     R2* pops2 = reinterpret_cast<R2*>(smem_raw);                  // [8][R1N] (cz = -1, cz = 0)
     R* pops1 = reinterpret_cast<R*>(pops2 + 8 * R1N);             // [8][R1N] (cz = +1)
-    R* phis = pops1 + 8 * R1N;                         // [PHI_SLOTS][R3N]     (TC)
+    R* phis = pops1 + 8 * R1N;                         // [PHI_SLOTS][R3N]
     auto gslot = [](int g) { return g < 4 ? g : g - 1; };  // shared slot of group g != 4
-    R* sxys = phis + (TC ? PHI_SLOTS * R3N : 0);       // [SXY_SLOTS][R2N]     (TC) S_x S_y phi
-    R* gxys = sxys + (TC ? SXY_SLOTS * R2N : 0);       // [GXY_SLOTS][2][R2N]  (TC) D_x S_y phi, S_x D_y phi
-    R* ths = gxys + (TC ? GXY_SLOTS * 2 * R2N : 0);    // [TH_SLOTS][3][R2N]   (TC) theta
-    R* gts = ths + (TC ? TH_SLOTS * 3 * R2N : 0);      // [GT_SLOTS][3][R1N]   (TC) g~
-    R* hs = gts + (TC ? GT_SLOTS * 3 * R1N : 0);       // [H_SLOTS][3][R1N]    (TC) theta partials
+    auto put_group = [&](int g, int node, R vm, R v0, R vp) {
+        R2 v;
+        v.x = vm;
+        v.y = v0;
+        pops2[gslot(g) * R1N + node] = v;
+        pops1[gslot(g) * R1N + node] = vp;
+    };
+    R* sxys = phis + PHI_SLOTS * R3N;       // [SXY_SLOTS][R2N] S_x S_y phi
+    R* gxys = sxys + SXY_SLOTS * R2N;       // [GXY_SLOTS][2][R2N] D_x S_y phi, S_x D_y phi
+    R* ths = gxys + GXY_SLOTS * 2 * R2N;    // [TH_SLOTS][3][R2N] theta
+    R* gts = ths + TH_SLOTS * 3 * R2N;      // [GT_SLOTS][3][R1N] g~
+    R* hs = gts + GT_SLOTS * 3 * R1N;       // [H_SLOTS][3][R1N] theta partials
 
     const int t = threadIdx.x;
     const int tx = t % TX, ty = t / TX;
@@ -158,7 +94,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     const long long N = p.N;
     const int plane = (int)p.plane;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const bool dr = TC && p.densratio;
+    const bool dr = p.densratio != 0;
     const bool obs = OBS && p.obstacles != 0;
     const R cssq = R(1.0 / 3.0);
 
@@ -209,7 +145,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     // phi mass correction of the input phi (compiled with the obstacle code only)
     double mcorr = 0.0;
     bool do_mcorr = false;
-    if constexpr (OBS && TC) do_mcorr = mass_corr(p.mass, mcorr);
+    if constexpr (OBS) do_mcorr = mass_corr(p.mass, mcorr);
     const int ox = X0 + tx, oy = Y0 + ty;
     const bool out_ok = (ox < nx) && (oy < ny);
     const int out_off = oy * nx + ox;
@@ -239,31 +175,29 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     }
     int r3_off[3] = {0, 0, 0};
     bool r3_ok[3] = {false, false, false};
-    if constexpr (TC) {
 #pragma unroll
-        for (int k = 0; k < KTH; ++k) {
-            int n = t + k * NTH;
-            if (t < NTH && n < R2N) {
-                int hx, hy;
-                r2_node(n, hx, hy);
-                bool ok = true;
-                int gx = wrap_coord(X0 + hx - 2, nx, p.pbx, ok);
-                int gy = wrap_coord(Y0 + hy - 2, ny, p.pby, ok);
-                r2_ok[k] = ok;
-                r2_off[k] = ok ? gy * nx + gx : 0;
-            }
+    for (int k = 0; k < KTH; ++k) {
+        int n = t + k * NTH;
+        if (t < NTH && n < R2N) {
+            int hx, hy;
+            r2_node(n, hx, hy);
+            bool ok = true;
+            int gx = wrap_coord(X0 + hx - 2, nx, p.pbx, ok);
+            int gy = wrap_coord(Y0 + hy - 2, ny, p.pby, ok);
+            r2_ok[k] = ok;
+            r2_off[k] = ok ? gy * nx + gx : 0;
         }
+    }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            int n = t + k * NT;
-            if (n < R3N) {
-                int hx = n % R3X, hy = n / R3X;
-                bool ok = true;
-                int gx = wrap_coord(X0 + hx - 3, nx, p.pbx, ok);
-                int gy = wrap_coord(Y0 + hy - 3, ny, p.pby, ok);
-                r3_ok[k] = ok;
-                r3_off[k] = ok ? gy * nx + gx : 0;
-            }
+    for (int k = 0; k < 3; ++k) {
+        int n = t + k * NT;
+        if (n < R3N) {
+            int hx = n % R3X, hy = n / R3X;
+            bool ok = true;
+            int gx = wrap_coord(X0 + hx - 3, nx, p.pbx, ok);
+            int gy = wrap_coord(Y0 + hy - 3, ny, p.pby, ok);
+            r3_ok[k] = ok;
+            r3_off[k] = ok ? gy * nx + gx : 0;
         }
     }
 
@@ -443,6 +377,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
         float v32[4];  // P, u, v, w of the 16-bit formats
         S uo[3];
         int8_t isf;
+        int row;  // start of the wall links of the warp's tile row
     };
     auto fetch = [&](int gi, NodeRaw& r) {
         if constexpr (LY::split) {
@@ -465,7 +400,9 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
         bool zk = true;
         const int wz = zwrap(q, zk);
         if (zk && okA) fetch(wz * plane + offA, nxt);
+        if (obs && q >= z0 && q < z1 && oy < ny) nxt.row = __ldg(p.link_rows + (q * ny + oy) * ((nx + TX - 1) / TX) + bx);
     };
+    nxt.row = 0;
 
     // accumulators of the raw moments {sum g, sum g c, sum g c c} for output planes
     // q-1 (am), q (a0), q+1 (ap); A2[i] = (am[i], a0[i]), one pair, accumulated
@@ -482,36 +419,34 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     }
 
     // ---- prologue: phi(z0-3..z0+2), theta(z0-2..z0) ----
-    if constexpr (TC) {
-        // partials of phi(z0-3..z0+1), theta(z0-2..z0), theta partials (z0-2, z0-1)
-        // (theta reads only this thread's own partials; the partial slots are
-        // reused as soon as a theta plane no longer needs them)
-        for (int q = z0 - 3; q <= z0 + 1; ++q) load_phi_plane(q, false);
-        __syncthreads();
-        planar_plane(z0 - 3);
-        planar_plane(z0 - 2);
-        planar_plane(z0 - 1);
-        if (obs) theta_isf(z0 - 2, th_isf);
-        theta_plane(z0 - 2);
-        planar_plane(z0);
-        if (obs) theta_isf(z0 - 1, th_isf);
-        theta_plane(z0 - 1);
-        planar_plane(z0 + 1);
-        __syncthreads();
-        theta_partials(z0 - 2);
-        theta_partials(z0 - 1);
-        __syncthreads();
-        if (obs) theta_isf(z0, th_isf);
-        theta_plane(z0);               // into the slot of theta(z0-2)
-        if (obs) theta_isf(z0 + 1, th_isf);  // for the loop's first theta plane
-        load_phi_plane(z0 + 2, true);  // into the slot of phi(z0-3), no longer read
-    }
+    // partials of phi(z0-3..z0+1), theta(z0-2..z0), theta partials (z0-2, z0-1)
+    // (theta reads only this thread's own partials; the partial slots are
+    // reused as soon as a theta plane no longer needs them)
+    for (int q = z0 - 3; q <= z0 + 1; ++q) load_phi_plane(q, false);
+    __syncthreads();
+    planar_plane(z0 - 3);
+    planar_plane(z0 - 2);
+    planar_plane(z0 - 1);
+    if (obs) theta_isf(z0 - 2, th_isf);
+    theta_plane(z0 - 2);
+    planar_plane(z0);
+    if (obs) theta_isf(z0 - 1, th_isf);
+    theta_plane(z0 - 1);
+    planar_plane(z0 + 1);
+    __syncthreads();
+    theta_partials(z0 - 2);
+    theta_partials(z0 - 1);
+    __syncthreads();
+    if (obs) theta_isf(z0, th_isf);
+    theta_plane(z0);               // into the slot of theta(z0-2)
+    if (obs) theta_isf(z0 + 1, th_isf);  // for the loop's first theta plane
+    load_phi_plane(z0 + 2, true);  // into the slot of phi(z0-3), no longer read
     prefetch_a(z0 - 1);
     cp_async_wait_all();
     __syncthreads();
     // theta partials of the first loop plane; the loop computes each later
     // plane's in the pull phase of the plane before
-    if constexpr (TC) theta_partials(z0);
+    theta_partials(z0);
 
     for (int q = z0 - 1; q <= z1; ++q) {
         bool zok = true;
@@ -522,10 +457,8 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
         // ================= phase 1 =================
         // partials of phi(q+3), then theta(q+2) from the partials of planes
         // q+1..q+3 (this thread's own nodes)
-        if constexpr (TC) {
-            planar_plane(q + 3);
-            theta_plane(q + 2);
-        }
+        planar_plane(q + 3);
+        theta_plane(q + 2);
 
         R c4m = R(0), c40 = R(0), c4p = R(0);  // centre group of the interior node
         // unrolled: the interior node's copy of the collision reads the
@@ -545,6 +478,10 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
             if (inb && obs) isf = cur.isf;
             const bool live = inb && (isf != 0);
             const bool interior = (k == 0) && out_ok && q_inner;
+            // the wall links of the interior node, loaded before its collision uses them
+            unsigned links = 0;
+            bool any_wall = false;
+            if (k == 0 && obs) links = wall_links(p, interior && isf == -1, cur.row, tx, any_wall);
             R fpop[27];
             bool ring_done = false;  // a ring node's populations are stored already
             R sP = 0, spxx = 0, spyy = 0, spzz = 0, spxy = 0, spxz = 0, spyz = 0, som = 0;
@@ -572,44 +509,42 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                 R phi = 0, lap = 0, divt = 0, gfx = 0, gfy = 0, gfz = 0;
                 R phi_u = 0;         // phi before the mass correction
                 bool stale = false;  // the collision reads phi_u (see below)
-                if constexpr (TC) {
-                    const int hx = node % R1X, hy = node / R1X;
-                    const int c2 = (hy + 1) * R2X + (hx + 1);
-                    const int c3 = (hy + 2) * R3X + (hx + 2);
-                    phi = phis[phi_slot(q) * R3N + c3];
-                    const R phm = phis[phi_slot(q - 1) * R3N + c3], php = phis[phi_slot(q + 1) * R3N + c3];
-                    const R* sm = sxys + sxy_slot(q - 1) * R2N;
-                    const R* s0 = sxys + sxy_slot(q) * R2N;
-                    const R* sp = sxys + sxy_slot(q + 1) * R2N;
-                    // S_z S_x S_y phi - phi, with W0 - 1 = -2 W1
-                    lap = R(6) * (W1 * (sm[c2] + sp[c2]) + W0 * s0[c2] + W1 * ((phm - phi) + (php - phi)));
-                    const R* hm = hs + h_slot(q - 1) * (3 * R1N);
-                    const R* h0 = hs + h_slot(q) * (3 * R1N);
-                    const R* hp = hs + h_slot(q + 1) * (3 * R1N);
-                    divt = R(3) * ((W1 * (hm[node] + hp[node]) + W0 * h0[node]) +
-                                   W1 * ((hp[R1N + node] - hm[R1N + node]) + (hp[2 * R1N + node] - hm[2 * R1N + node])));
-                    const R* g1 = gts + gt_slot(q) * (3 * R1N);
-                    gfx = g1[0 * R1N + node];
-                    gfy = g1[1 * R1N + node];
-                    gfz = g1[2 * R1N + node];
-                    if constexpr (OBS) {
-                        // from here on the input phi after the mass correction (the
-                        // gradient, theta and Laplacian above are compute_norm's, from
-                        // the uncorrected phi)
-                        if (do_mcorr) {
-                            phi_u = phi;
-                            phi = (R)mass_corrected<SP>((double)phi, mcorr);
-                            // a node reached across a periodic face is, in the
-                            // reference's fused kernel, a halo copy: its moments and
-                            // forces were exchanged after the moments kernel (corrected
-                            // phi), its phi before the correction
-                            stale = phi != phi_u && ((k ? wrapB : wrapA) || q < 0 || q >= nz);
-                        }
+                const int hx = node % R1X, hy = node / R1X;
+                const int c2 = (hy + 1) * R2X + (hx + 1);
+                const int c3 = (hy + 2) * R3X + (hx + 2);
+                phi = phis[phi_slot(q) * R3N + c3];
+                const R phm = phis[phi_slot(q - 1) * R3N + c3], php = phis[phi_slot(q + 1) * R3N + c3];
+                const R* sm = sxys + sxy_slot(q - 1) * R2N;
+                const R* s0 = sxys + sxy_slot(q) * R2N;
+                const R* sp = sxys + sxy_slot(q + 1) * R2N;
+                // S_z S_x S_y phi - phi, with W0 - 1 = -2 W1
+                lap = R(6) * (W1 * (sm[c2] + sp[c2]) + W0 * s0[c2] + W1 * ((phm - phi) + (php - phi)));
+                const R* hm = hs + h_slot(q - 1) * (3 * R1N);
+                const R* h0 = hs + h_slot(q) * (3 * R1N);
+                const R* hp = hs + h_slot(q + 1) * (3 * R1N);
+                divt = R(3) * ((W1 * (hm[node] + hp[node]) + W0 * h0[node]) +
+                               W1 * ((hp[R1N + node] - hm[R1N + node]) + (hp[2 * R1N + node] - hm[2 * R1N + node])));
+                const R* g1 = gts + gt_slot(q) * (3 * R1N);
+                gfx = g1[0 * R1N + node];
+                gfy = g1[1 * R1N + node];
+                gfz = g1[2 * R1N + node];
+                if constexpr (OBS) {
+                    // from here on the input phi after the mass correction (the
+                    // gradient, theta and Laplacian above are compute_norm's, from
+                    // the uncorrected phi)
+                    if (do_mcorr) {
+                        phi_u = phi;
+                        phi = (R)mass_corrected<SP>((double)phi, mcorr);
+                        // a node reached across a periodic face is, in the
+                        // reference's fused kernel, a halo copy: its moments and
+                        // forces were exchanged after the moments kernel (corrected
+                        // phi), its phi before the correction
+                        stale = phi != phi_u && ((k ? wrapB : wrapA) || q < 0 || q >= nz);
                     }
                 }
                 // ---- moments prologue: lb_cuda_moments_module.f90:104-339 ----
                 R inv = R(1), mask = R(0), fxv, fyv, fzv;
-                if constexpr (TC) mask = R(4) * phi * (R(1) - phi);
+                mask = R(4) * phi * (R(1) - phi);
                 if (dr) {
                     const R rhophi = p.rho_r * phi + (R(1) - phi) * p.rho_b;
                     inv = rcp<R>(rhophi);
@@ -619,24 +554,22 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                 }
                 R grx = 0, gry = 0, grz = 0, cv = 0, omega;
                 R visc_l = p.visc1;  // local viscosity (mixture with two components)
-                if constexpr (TC) {
-                    const R chem = R(4) * p.beta * phi * (phi - R(1)) * (phi - R(0.5)) - p.kapp * lap;
-                    fxv += chem * gfx;
-                    fyv += chem * gfy;
-                    fzv += chem * gfz;
-                    if constexpr (REP) {
-                        // REPULSIVE_FLUX (lb_cuda_moments_module.f90:148-160): rho_phi F_rep,
-                        // each component capped at 1e-3, times rho_phi
-                        const R rh = dr ? p.rho_r * phi + (R(1) - phi) * p.rho_b : R(1);
-                        const R cap = R(1.0e-3);
-                        R t0 = p.rep[gi] * rh, t1 = p.rep[N + gi] * rh, t2 = p.rep[2 * N + gi] * rh;
-                        t0 = t0 > cap ? cap : (t0 < -cap ? -cap : t0);
-                        t1 = t1 > cap ? cap : (t1 < -cap ? -cap : t1);
-                        t2 = t2 > cap ? cap : (t2 < -cap ? -cap : t2);
-                        fxv += t0 * rh;
-                        fyv += t1 * rh;
-                        fzv += t2 * rh;
-                    }
+                const R chem = R(4) * p.beta * phi * (phi - R(1)) * (phi - R(0.5)) - p.kapp * lap;
+                fxv += chem * gfx;
+                fyv += chem * gfy;
+                fzv += chem * gfz;
+                if constexpr (REP) {
+                    // REPULSIVE_FLUX (lb_cuda_moments_module.f90:148-160): rho_phi F_rep,
+                    // each component capped at 1e-3, times rho_phi
+                    const R rh = dr ? p.rho_r * phi + (R(1) - phi) * p.rho_b : R(1);
+                    const R cap = R(1.0e-3);
+                    R t0 = p.rep[gi] * rh, t1 = p.rep[N + gi] * rh, t2 = p.rep[2 * N + gi] * rh;
+                    t0 = t0 > cap ? cap : (t0 < -cap ? -cap : t0);
+                    t1 = t1 > cap ? cap : (t1 < -cap ? -cap : t1);
+                    t2 = t2 > cap ? cap : (t2 < -cap ? -cap : t2);
+                    fxv += t0 * rh;
+                    fyv += t1 * rh;
+                    fzv += t2 * rh;
                 }
                 if (dr) {
                     const R drho = p.rho_r - p.rho_b;
@@ -672,13 +605,9 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                     u += R(0.5) * fxv * inv;
                     v += R(0.5) * fyv * inv;
                     w += R(0.5) * fzv * inv;
-                    if constexpr (TC) {
-                        const R visc = (p.rho_r * p.visc1 * phi + (R(1) - phi) * p.visc2 * p.rho_b) * inv;
-                        visc_l = visc;
-                        omega = rcp<R>(visc * R(3) + R(0.5));
-                    } else {
-                        omega = p.omega;
-                    }
+                    const R visc = (p.rho_r * p.visc1 * phi + (R(1) - phi) * p.visc2 * p.rho_b) * inv;
+                    visc_l = visc;
+                    omega = rcp<R>(visc * R(3) + R(0.5));
                 }
                 pxx += fxv * u * inv;
                 pyy += fyv * v * inv;
@@ -700,14 +629,12 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                         CD::st(p.uout + 1 * N, gi, v, p.scale[F_UOLD + 1]);
                         CD::st(p.uout + 2 * N, gi, w, p.scale[F_UOLD + 2]);
                     }
-                    if constexpr (TC) {
-                        // update_phifields: lb_cuda_update_phi_module.f90:77-93
-                        const R phi_new = phi - u * R(0.5) * gfx - v * R(0.5) * gfy - w * R(0.5) * gfz +
-                                          p.tau_diff * lap - p.sharp_c * divt;
-                        CP::st(p.pout, gi, phi_new, p.scale[F_PHI]);
-                    }
+                    // update_phifields: lb_cuda_update_phi_module.f90:77-93
+                    const R phi_new = phi - u * R(0.5) * gfx - v * R(0.5) * gfy - w * R(0.5) * gfz +
+                                      p.tau_diff * lap - p.sharp_c * divt;
+                    CP::st(p.pout, gi, phi_new, p.scale[F_PHI]);
                 }
-                if constexpr (OBS && TC) {
+                if constexpr (OBS) {
                     if (stale) {
                         // density and viscosity of the collision from the halo copy's
                         // uncorrected phi (lb_cuda_fused_module.f90:590-620)
@@ -748,146 +675,29 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                     M[2][0][0] = mxx; M[0][2][0] = myy; M[0][0][2] = mzz;
                     M[1][1][0] = mxy; M[1][0][1] = mxz; M[0][1][1] = myz;
                     if constexpr (HO) {
-                        const R X = Xn, Y = Yn, Z = Zn, XY = XYn, XZ = XZn, YZ = YZn;
-                        const R u2 = u * u, v2 = v * v, w2 = w * w;
-                        // rows 10..26 of the reference (lb_cuda_fused_module.f90:667-703)
-                        M[2][1][0] = u2 * v + om1 * (R(2) * XY * u + X * v);
-                        M[2][0][1] = u2 * w + om1 * (R(2) * XZ * u + X * w);
-                        M[1][2][0] = u * v2 + om1 * (Y * u + R(2) * XY * v);
-                        M[1][0][2] = u * w2 + om1 * (Z * u + R(2) * XZ * w);
-                        M[0][1][2] = v * w2 + om1 * (Z * v + R(2) * YZ * w);
-                        M[0][2][1] = v2 * w + om1 * (R(2) * YZ * v + Y * w);
-                        M[1][1][1] = u * v * w + om1 * (YZ * u + XZ * v + XY * w);
-                        M[2][2][0] = u2 * v2 + om1 * (Y * u2 + R(2) * v * (R(3) * XY * u + X * v));
-                        M[2][0][2] = u2 * w2 + om1 * (Z * u2 + R(2) * w * (R(3) * XZ * u + X * w));
-                        M[0][2][2] = v2 * w2 + om1 * (Z * v2 + R(2) * w * (R(3) * YZ * v + Y * w));
-                        M[1][1][2] = u * v * w2 + om1 * (Z * u * v + w * (R(3) * YZ * u + R(3) * XZ * v + R(2) * XY * w));
-                        M[1][2][1] = u * v2 * w +
-                                     om1 * (R(2) * YZ * u * v + XZ * v2 + R(2) * Y * u * w + R(4) * XY * v * w);
-                        M[2][1][1] = u2 * v * w +
-                                     om1 * (YZ * u2 + R(2) * XZ * u * v + R(4) * XY * u * w + R(2) * X * v * w);
-                        M[2][1][2] = u2 * v * w2 + om1 * (Z * u2 * v + R(3) * w * (YZ * u2 + R(2) * XZ * u * v +
-                                                                                 R(2) * XY * u * w + X * v * w));
-                        M[2][2][1] = u2 * v2 * w + om1 * (R(2) * u * v * (YZ * u + XZ * v) + R(2) * Y * u2 * w +
-                                                          v * (R(10) * XY * u + R(3) * X * v) * w);
-                        M[1][2][2] = u * v2 * w2 + om1 * (Z * u * v2 + R(3) * w * (R(2) * YZ * u * v + XZ * v2 +
-                                                                                  Y * u * w + R(2) * XY * v * w));
-                        M[2][2][2] = u2 * v2 * w2 +
-                                     om1 * (Z * u2 * v2 + w * (R(6) * u * v * (YZ * u + XZ * v) + R(3) * Y * u2 * w +
-                                                               R(2) * v * (R(7) * XY * u + R(2) * X * v) * w));
+                        ho_rows<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
                     } else {
                         M[2][1][0] = M[2][0][1] = M[1][2][0] = M[1][0][2] = M[0][1][2] = M[0][2][1] = M[1][1][1] = R(0);
                         M[2][2][0] = M[2][0][2] = M[0][2][2] = M[1][1][2] = M[1][2][1] = M[2][1][1] = R(0);
                         M[2][1][2] = M[2][2][1] = M[1][2][2] = M[2][2][2] = R(0);
                     }
-                    if (k == 1 && ring_col) {
-                        // column ring node: the x transform at cx = ring_dir only,
-                        // the same operations as the full transform for that value
-                        R T[3][3];  // [b][c]
-#pragma unroll
-                        for (int b = 0; b < 3; ++b)
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                const R sv = fmaf_t(M[0][b][c], R(1.0 / 6.0), R(0.5) * M[2][b][c]);
-                                T[b][c] = sv + ring_dir * (R(0.5) * M[1][b][c]);
-                            }
-                        R Y[3][3];  // [b][c]
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) d1q3_inv<R>(T[0][c], T[1][c], T[2][c], Y[0][c], Y[1][c], Y[2][c]);
-                        const int xg = ring_dir > R(0) ? 2 : 0;
-#pragma unroll
-                        for (int b = 0; b < 3; ++b) {
-                            R vm, v0, vp;
-                            d1q3_inv<R>(Y[b][0], Y[b][1], Y[b][2], vm, v0, vp);
-                            R2 v2;
-                            v2.x = vm;
-                            v2.y = v0;
-                            pops2[gslot(3 * b + xg) * R1N + node] = v2;
-                            pops1[gslot(3 * b + xg) * R1N + node] = vp;
-                        }
-                        ring_done = true;
+                    if (k == 0) {
+                        full_pops27<R>(M, fpop);
                     } else {
-                        // the x (a) and y (b) transforms packed over the pair
-                        // c = 0, 1 of the z coefficient index, c = 2 alone; both
-                        // take the second coefficient negated, carried by the
-                        // sign (-1)^([a==2] + [b==2]) of the coefficients (exact:
-                        // the values are those of the scalar transforms)
-                        using PT = typename PK<R>::T;
-                        PT P[3][3];
-                        R Q[3][3];
-#pragma unroll
-                        for (int a = 0; a < 3; ++a)
-#pragma unroll
-                            for (int b = 0; b < 3; ++b) {
-                                const R sg = ((a == 2) != (b == 2)) ? R(-1) : R(1);
-                                P[a][b] = PK<R>::mk(sg * M[a][b][0], sg * M[a][b][1]);
-                                Q[a][b] = sg * M[a][b][2];
-                            }
-                        // x transform: TP/TQ[a'][b], with the sign (-1)^[b==2]
-                        PT TP[3][3];
-                        R TQ[3][3];
-#pragma unroll
-                        for (int b = 0; b < 3; ++b) {
-                            d1q3n2<R>(P[0][b], P[1][b], P[2][b], TP[0][b], TP[1][b], TP[2][b]);
-                            d1q3n<R>(Q[0][b], Q[1][b], Q[2][b], TQ[0][b], TQ[1][b], TQ[2][b]);
-                        }
-                        if (k == 1) {
-                            // row ring node: the y transform at cy = ring_dir only
-                            const int yg = ring_dir > R(0) ? 2 : 0;
-#pragma unroll
-                            for (int a = 0; a < 3; ++a) {
-                                R Y[3];
-#pragma unroll
-                                for (int c = 0; c < 3; ++c) {
-                                    const R t0 = c == 0 ? TP[a][0].x : (c == 1 ? TP[a][0].y : TQ[a][0]);
-                                    const R t1 = c == 0 ? TP[a][1].x : (c == 1 ? TP[a][1].y : TQ[a][1]);
-                                    const R t2n = c == 0 ? TP[a][2].x : (c == 1 ? TP[a][2].y : TQ[a][2]);
-                                    const R sv = fmaf_t(t0, R(1.0 / 6.0), R(-0.5) * t2n);
-                                    Y[c] = sv + ring_dir * (R(0.5) * t1);
-                                }
-                                R vm, v0, vp;
-                                d1q3_inv<R>(Y[0], Y[1], Y[2], vm, v0, vp);
-                                R2 v2;
-                                v2.x = vm;
-                                v2.y = v0;
-                                pops2[gslot(3 * yg + a) * R1N + node] = v2;
-                                pops1[gslot(3 * yg + a) * R1N + node] = vp;
-                            }
-                            ring_done = true;
-                        } else {
-                            // y transform: MP/MQ[a][b'], then the z transform scalar
-                            PT MP[3][3];
-                            R MQ[3][3];
-#pragma unroll
-                            for (int a = 0; a < 3; ++a) {
-                                d1q3n2<R>(TP[a][0], TP[a][1], TP[a][2], MP[a][0], MP[a][1], MP[a][2]);
-                                d1q3n<R>(TQ[a][0], TQ[a][1], TQ[a][2], MQ[a][0], MQ[a][1], MQ[a][2]);
-                            }
-#pragma unroll
-                            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                                for (int b = 0; b < 3; ++b) {
-                                    R vm, v0, vp;
-                                    d1q3_inv<R>(MP[a][b].x, MP[a][b].y, MQ[a][b], vm, v0, vp);
-                                    fpop[LINK(a - 1, b - 1, -1)] = vm;
-                                    fpop[LINK(a - 1, b - 1, 0)] = v0;
-                                    fpop[LINK(a - 1, b - 1, 1)] = vp;
-                                }
-                        }
+                        // a ring node's populations go to shared memory at once
+                        const bool plus = ring_dir > R(0);
+                        if (ring_col)
+                            ring_col_pops27<R>(M, ring_dir, [&](int b, R vm, R v0, R vp) {
+                                put_group(3 * b + (plus ? 2 : 0), node, vm, v0, vp);
+                            });
+                        else
+                            ring_row_pops27<R>(M, ring_dir, [&](int a, R vm, R v0, R vp) {
+                                put_group(3 * (plus ? 2 : 0) + a, node, vm, v0, vp);
+                            });
+                        ring_done = true;
                     }
                 } else {
-                    // D3Q19 / D3Q15: the second-order expansion link by link (D3Q27 indices)
-                    const R base = m0 - R(1.5) * (mxx + myy + mzz);
-#pragma unroll
-                    for (int l = 0; l < 27; ++l) {
-                        if (!IN<LAT>(l)) continue;
-                        const int cx = EX(l), cy = EY(l), cz = EZ(l);
-                        R s = base;
-                        s += R(3) * (R(cx) * mx + R(cy) * my + R(cz) * mz);
-                        s += R(4.5) * (R(cx * cx) * mxx + R(cy * cy) * myy + R(cz * cz) * mzz);
-                        s += R(9) * (R(cx * cy) * mxy + R(cx * cz) * mxz + R(cy * cz) * myz);
-                        fpop[l] = R(WL<LAT>(l)) * s;
-                    }
+                    low_order_pops<LAT, R>(m0, mx, my, mz, mxx, myy, mzz, mxy, mxz, myz, fpop);
                 }
             } else {
 #pragma unroll
@@ -916,43 +726,11 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
             }
 
             // ---- obstacle bounce-back: lb_cuda_boundary_module.f90:162-199 ----
-            if (interior && obs && isf == -1) {
-                const R om1 = R(1) - som;
-                // neighbour x / y coordinates of the output node, computed here:
-                // held in registers through the whole sweep they cost the
-                // obstacle step 4 registers at its limit of 128 and 10.7 % of
-                // its time on a box with obstacles
-                int nbx[3], nby[3];
-                bool nbx_ok[3], nby_ok[3];
+            if (k == 0 && any_wall) {
+                R d[10];
+                wall_link_sums<LAT, R>(links, sP, R(1) - som, spxx, spyy, spzz, spxy, spxz, spyz, d);
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    bool okx = true, oky = true;
-                    nbx[d] = wrap_coord(ox + d - 1, nx, p.pbx, okx);
-                    nby[d] = wrap_coord(oy + d - 1, ny, p.pby, oky);
-                    nbx_ok[d] = okx;
-                    nby_ok[d] = oky;
-                }
-#pragma unroll
-                for (int l = 1; l < 27; ++l) {
-                    if (!IN<LAT>(l)) continue;
-                    const int cx = EX(l), cy = EY(l), cz = EZ(l);
-                    const int ix = 1 - cx, iy = 1 - cy;
-                    bool zk = true;
-                    const int zz = zwrap(q - cz, zk);
-                    int s = 1;
-                    if (nbx_ok[ix] && nby_ok[iy] && zk) s = p.isf[zz * plane + nby[iy] * nx + nbx[ix]];
-                    if (s != 0) continue;
-                    const R wl = R(WL<LAT>(l));
-                    const R dx = R(cx), dy = R(cy), dz = R(cz);
-                    const R fneq = wl * R(4.5) *
-                                   ((dx * dx - cssq) * spxx + (dy * dy - cssq) * spyy + (dz * dz - cssq) * spzz +
-                                    R(2) * (dx * dy) * spxy + R(2) * (dx * dz) * spxz + R(2) * (dy * dz) * spyz);
-                    const R fp = wl * sP + om1 * fneq;
-                    A2[0].y += fp;
-                    A2[1].y += fp * dx; A2[2].y += fp * dy; A2[3].y += fp * dz;
-                    A2[4].y += fp * (dx * dx); A2[5].y += fp * (dy * dy); A2[6].y += fp * (dz * dz);
-                    A2[7].y += fp * (dx * dy); A2[8].y += fp * (dx * dz); A2[9].y += fp * (dy * dz);
-                }
+                for (int i = 0; i < 10; ++i) A2[i].y += d[i];
             }
         }
         // the interior node's fields of plane q+1, issued before the barrier
@@ -962,15 +740,15 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
 
         // ================= phase 2 =================
         // the slot of phi(q-1) was last read in phase 1
-        if constexpr (TC) load_phi_plane(q + 4, true);
-        if (TC && obs) theta_isf(q + 3, th_isf);  // for theta(q+3), next plane
+        load_phi_plane(q + 4, true);
+        if (obs) theta_isf(q + 3, th_isf);  // for theta(q+3), next plane
         // the theta partials of plane q+2 at this thread's collision nodes
         // (theta(q+2) is complete since the barrier after phase 1).  Here
         // rather than in phase 1 they fill the shorter pull phase and shorten
         // the collision phase, whose barrier waits for the ring collisions
         // (1.7 % per step at 256^3); before the pull rather than after it,
         // 0.3 % more
-        if constexpr (TC) theta_partials(q + 2);
+        theta_partials(q + 2);
 
         // the three cz populations of every (cx, cy) group from node x - c:
         // cz = -1, 0 as one pair (packed sums), cz = +1 alone
@@ -992,77 +770,11 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                 gp[yc][xc] = PK<R>::mk(v.x, v.y);
                 gs[yc][xc] = pops1[gslot(g) * R1N + src];
             }
-        {
-            using P = PK<R>;
-            const PP m1 = P::mk(R(-1), R(-1));
-            PP S0[3], S1[3], S2[3];
-#pragma unroll
-            for (int yc = 0; yc < 3; ++yc) {
-                const PP* g = gp[yc];
-                S0[yc] = P::add(P::add(g[0], g[1]), g[2]);
-                S1[yc] = P::fma(g[0], m1, g[2]);
-                S2[yc] = P::add(g[2], g[0]);
-            }
-            const PP Y00 = P::add(P::add(S0[0], S0[1]), S0[2]);
-            const PP Y01 = P::fma(S0[0], m1, S0[2]);
-            const PP Y02 = P::add(S0[2], S0[0]);
-            const PP Y10 = P::add(P::add(S1[0], S1[1]), S1[2]);
-            const PP Y11 = P::fma(S1[0], m1, S1[2]);
-            const PP Y20 = P::add(P::add(S2[0], S2[1]), S2[2]);
-            // accum_slice for cz = -1 (x) and 0 (y)
-            const PP cz = P::mk(R(-1), R(0)), cz2 = P::mk(R(1), R(0));
-            A2[0] = P::add(A2[0], Y00);
-            A2[1] = P::add(A2[1], Y10);
-            A2[2] = P::add(A2[2], Y01);
-            A2[3] = P::fma(cz, Y00, A2[3]);
-            A2[4] = P::add(A2[4], Y20);
-            A2[5] = P::add(A2[5], Y02);
-            A2[6] = P::fma(cz2, Y00, A2[6]);
-            A2[7] = P::add(A2[7], Y11);
-            A2[8] = P::fma(cz, Y10, A2[8]);
-            A2[9] = P::fma(cz, Y01, A2[9]);
-        }
-        {
-            R S0[3], S1[3], S2[3];
-#pragma unroll
-            for (int yc = 0; yc < 3; ++yc) {
-                const R* g = gs[yc];
-                S0[yc] = g[0] + g[1] + g[2];
-                S1[yc] = g[2] - g[0];
-                S2[yc] = g[2] + g[0];
-            }
-            const R Y00 = S0[0] + S0[1] + S0[2];
-            const R Y01 = S0[2] - S0[0];
-            const R Y02 = S0[2] + S0[0];
-            const R Y10 = S1[0] + S1[1] + S1[2];
-            const R Y11 = S1[2] - S1[0];
-            const R Y20 = S2[0] + S2[1] + S2[2];
-            accum_slice<R>(ap, R(1), Y00, Y01, Y02, Y10, Y11, Y20);
-        }
+        pull_sums27<R>(gp, gs, A2, ap);
         R am[10];
 #pragma unroll
         for (int i = 0; i < 10; ++i) am[i] = A2[i].x;
-        if (q - 1 >= z0 && out_ok) {
-            const int go = (q - 1) * plane + out_off;
-            const R third = am[0] * cssq;
-            if constexpr (CD::scaled) {
-                am[4] -= am[1] * am[1]; am[5] -= am[2] * am[2]; am[6] -= am[3] * am[3];
-                am[7] -= am[1] * am[2]; am[8] -= am[1] * am[3]; am[9] -= am[2] * am[3];
-            }
-            if constexpr (LY::split) {
-#pragma unroll
-                for (int f = 0; f < 4; ++f) p.pres_out[f * N + go] = (float)am[f];
-            } else {
-#pragma unroll
-                for (int f = 0; f < 4; ++f) CD::st(p.mout + f * N, go, am[f], p.scale[f]);
-            }
-            CD::st(p.mout + LY::off(4, N), go, am[4] - third, p.scale[4]);
-            CD::st(p.mout + LY::off(5, N), go, am[5] - third, p.scale[5]);
-            CD::st(p.mout + LY::off(6, N), go, am[6] - third, p.scale[6]);
-            CD::st(p.mout + LY::off(7, N), go, am[7], p.scale[7]);
-            CD::st(p.mout + LY::off(8, N), go, am[8], p.scale[8]);
-            CD::st(p.mout + LY::off(9, N), go, am[9], p.scale[9]);
-        }
+        if (q - 1 >= z0 && out_ok) write_moments<S, R>(p, (q - 1) * plane + out_off, am);
 #pragma unroll
         for (int i = 0; i < 10; ++i) {
             A2[i] = PK<R>::mk(A2[i].y, ap[i]);
@@ -1073,8 +785,20 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     }
 }
 
-// CTAs per SM the kernel is compiled for: two of 256 threads, one of 512, one in FP64
+// CTAs per SM the kernel is compiled for: two of 8-row tiles, one of 16 rows, one in FP64
 template <typename R, int TYV> constexpr int step_min_blocks() { return (sizeof(R) == 8 || TYV > 8) ? 1 : 2; }
+
+// threads and shared memory of a CTA, by component class
+template <bool TC, int TYV> constexpr int step_threads() { return TC ? TX * TYV : single_threads<TYV>(); }
+template <int LAT, bool TC, typename S, typename R, int TYV> constexpr size_t step_smem_bytes() {
+    if constexpr (TC) return stream_smem_bytes<S, R, TYV>();
+    else return single_smem_bytes<LAT, R, TYV>();
+}
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP, bool OBS>
+__device__ __forceinline__ void any_body(const StepParams<S, R>& p, int bx, int by, int z0, int z1) {
+    if constexpr (TC) step_body<LAT, HO, S, R, TYV, REP, OBS>(p, bx, by, z0, z1);
+    else single_body<LAT, HO, S, R, TYV, OBS>(p, bx, by, z0, z1);
+}
 
 // Column-planes of the planes zlo .. zlo + nzr - 1 of a box for a tile of
 // TYV rows, column index = by * gx + bx, plane fastest.
@@ -1105,7 +829,7 @@ __device__ __forceinline__ void run_share(const int nx, const int nzr, const int
 // separately inlined copies may contract floating-point operations
 // differently and give results that differ in the last bit.
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
-__global__ void __launch_bounds__(TX * TYV, step_min_blocks<R, TYV>()) stream_kernel(const StepParams<S, R> p) {
+__global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>()) stream_kernel(const StepParams<S, R> p) {
     long long s0, s1;
     const int nzr = p.zhi - p.zlo;
     if (p.zseg < 0) {
@@ -1127,7 +851,7 @@ __global__ void __launch_bounds__(TX * TYV, step_min_blocks<R, TYV>()) stream_ke
         s1 = min(W, s0 + share);
     }
     run_share<TYV>(p.nx, nzr, p.zlo, s0, s1,
-                   [&](int bx, int by, int z0, int z1) { step_body<LAT, HO, TC, S, R, TYV, REP, OBS>(p, bx, by, z0, z1); });
+                   [&](int bx, int by, int z0, int z1) { any_body<LAT, HO, TC, S, R, TYV, REP, OBS>(p, bx, by, z0, z1); });
 }
 
 // Many boxes in one launch: CTA i advances box work[i].x over column-planes
@@ -1135,14 +859,14 @@ __global__ void __launch_bounds__(TX * TYV, step_min_blocks<R, TYV>()) stream_ke
 // box's own parameters and fields.  Each node's arithmetic is the same as in
 // stream_kernel, so a box gives the same bits alone and in a batch.
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
-__global__ void __launch_bounds__(TX * TYV, step_min_blocks<R, TYV>())
+__global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>())
     stream_kernel_batched(const StepParams<S, R>* __restrict__ boxes, const int4* __restrict__ work) {
     __shared__ StepParams<S, R> sp;
     const int4 w = work[blockIdx.x];
     if (threadIdx.x == 0) sp = boxes[w.x];
     __syncthreads();
     run_share<TYV>(sp.nx, sp.nz, 0, w.y, w.z,
-                   [&](int bx, int by, int z0, int z1) { step_body<LAT, HO, TC, S, R, TYV, REP, OBS>(sp, bx, by, z0, z1); });
+                   [&](int bx, int by, int z0, int z1) { any_body<LAT, HO, TC, S, R, TYV, REP, OBS>(sp, bx, by, z0, z1); });
 }
 
 }  // namespace lbf

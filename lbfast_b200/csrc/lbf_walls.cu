@@ -11,7 +11,7 @@
 #include <type_traits>
 
 #include "lbf_internal.h"
-#include "lbf_stream_kernel.cuh"
+#include "lbf_node.cuh"
 
 namespace lbf {
 namespace {
