@@ -166,7 +166,7 @@ std::map<TuneKey, std::pair<int, int>> g_tune_cache;
 TuneKey tune_key(const lbf_handle* h) {
     const lbf_params& p = h->p;
     return TuneKey{{p.storage, p.lattice, p.highorder, p.twocomponent, p.densratio, p.obstacles, p.lx, p.ly, p.lz,
-                    p.pbc_x * 4 + p.pbc_y * 2 + p.pbc_z, p.zseg, 0}};
+                    p.pbc_x * 4 + p.pbc_y * 2 + p.pbc_z, p.zseg, p.phi_correction != 0}};
 }
 
 int autotune(lbf_handle* h) {

@@ -45,7 +45,7 @@ template <typename S, typename R> void make_params(const StepArgs& a, StepParams
     p.mass = a.mass;
 }
 
-template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
 cudaError_t launch_stream(const StepArgs& a, cudaStream_t st) {
     static bool attr_set = false;
     const size_t smem = step_smem_bytes<LAT, TC, S, R, TYV>();
@@ -86,7 +86,7 @@ cudaError_t launch_stream(const StepArgs& a, cudaStream_t st) {
 // One launch advancing many boxes of one kernel class: d_boxes holds one
 // StepParams per box, d_work one (box, first column-plane, end column-plane)
 // per CTA.
-template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
 cudaError_t launch_stream_batched(const void* d_boxes, const int4* d_work, int nwork, cudaStream_t st) {
     static bool attr_set = false;
     const size_t smem = step_smem_bytes<LAT, TC, S, R, TYV>();
@@ -102,7 +102,7 @@ cudaError_t launch_stream_batched(const void* d_boxes, const int4* d_work, int n
     return cudaGetLastError();
 }
 
-template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true> int batched_resident() {
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1> int batched_resident() {
     static int resident = 0;
     if (!resident) {
         const size_t smem = step_smem_bytes<LAT, TC, S, R, TYV>();
@@ -121,15 +121,18 @@ template <typename S, typename R> void fill_params(const StepArgs& a, void* dst)
 }
 
 // the kernel classes of one storage type and tile height; tc: 0 one
-// component, 1 two components, 2 two components with REPULSIVE_FLUX; obs:
-// obstacles
-template <int LAT, bool HO, typename S, typename R, int TYV, bool OBS> StepLauncher step_class(int tc) {
+// component, 1 two components, 2 two components with REPULSIVE_FLUX; obs: see
+// kernel_obs
+template <int LAT, bool HO, typename S, typename R, int TYV, int OBS> StepLauncher step_class(int tc) {
     return tc == 2 ? &launch_stream<LAT, HO, true, S, R, TYV, true, OBS>
                    : tc ? &launch_stream<LAT, HO, true, S, R, TYV, false, OBS>
                         : &launch_stream<LAT, HO, false, S, R, TYV, false, OBS>;
 }
 template <int LAT, bool HO, typename S, typename R, int TYV> StepLauncher step_class(int tc, int obs) {
-    return obs ? step_class<LAT, HO, S, R, TYV, true>(tc) : step_class<LAT, HO, S, R, TYV, false>(tc);
+    // the correction without obstacles and without REPULSIVE_FLUX is a class of
+    // its own; with REPULSIVE_FLUX the obstacle compilation serves
+    if (obs == 2 && tc == 1) return &launch_stream<LAT, HO, true, S, R, TYV, false, 2>;
+    return obs ? step_class<LAT, HO, S, R, TYV, 1>(tc) : step_class<LAT, HO, S, R, TYV, 0>(tc);
 }
 template <typename S, typename R, int TYV> StepLauncher step_table(int lat, int ho, int tc, int obs) {
     if (lat == 15 && !ho) return step_class<15, false, S, R, TYV>(tc, obs);
@@ -139,7 +142,7 @@ template <typename S, typename R, int TYV> StepLauncher step_table(int lat, int 
     return nullptr;
 }
 
-template <int LAT, bool HO, typename S, typename R, int TYV, bool OBS> void batch_class(int tc, BatchOps& o) {
+template <int LAT, bool HO, typename S, typename R, int TYV, int OBS> void batch_class(int tc, BatchOps& o) {
     if (tc == 2) {
         o.launch = &launch_stream_batched<LAT, HO, true, S, R, TYV, true, OBS>;
         o.resident = &batched_resident<LAT, HO, true, S, R, TYV, true, OBS>;
@@ -151,12 +154,12 @@ template <int LAT, bool HO, typename S, typename R, int TYV, bool OBS> void batc
         o.resident = &batched_resident<LAT, HO, false, S, R, TYV, false, OBS>;
     }
 }
-// The batched kernels keep obstacles a run-time flag (OBS = true for every
+// The batched kernels keep obstacles a run-time flag (OBS = 1 for every
 // box): the obstacle-free compilation of the batched kernel, unlike the
 // single-box one, ran the droplet-ensemble server slower and erratically
 // (3.2-5.2 against a steady 5.5 solves/s, interleaved runs on one box).
 template <int LAT, bool HO, typename S, typename R, int TYV> void batch_class(int tc, int, BatchOps& o) {
-    batch_class<LAT, HO, S, R, TYV, true>(tc, o);
+    batch_class<LAT, HO, S, R, TYV, 1>(tc, o);
 }
 template <typename S, typename R, int TYV> BatchOps batch_table(int lat, int ho, int tc, int obs) {
     BatchOps o;

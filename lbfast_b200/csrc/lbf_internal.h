@@ -41,9 +41,10 @@ StepLauncher step_launcher(int storage, int lat, int ho, int tc, int obs, int ti
 // kernel class argument `tc` of a run: 0 one component, 1 two components,
 // 2 two components with REPULSIVE_FLUX (its own compilation of the step)
 inline int kernel_tc(const lbf_params& p) { return p.twocomponent ? (p.repulsive_flux ? 2 : 1) : 0; }
-// kernel class argument `obs`: the compilation with the obstacle code, which
-// also carries the phi mass correction of the step's input phi
-inline int kernel_obs(const lbf_params& p) { return (p.obstacles || p.phi_correction) ? 1 : 0; }
+// kernel class argument `obs`: 1 the compilation with the obstacle code, which
+// also carries the phi mass correction of the step's input phi, 2 the
+// correction without obstacles, 0 neither
+inline int kernel_obs(const lbf_params& p) { return p.obstacles ? 1 : p.phi_correction ? 2 : 0; }
 bool tile_available(int storage, int tile_y);
 
 // Batched step of many boxes of one kernel class and tile height: fill writes

@@ -1,6 +1,7 @@
 // lbf_misc.cu -- the small kernels around the fused step: wetting ghost phi,
 // field conversions at the host boundary, copy_print extraction and FP64
 // reductions.
+#include <algorithm>
 #include <type_traits>
 
 #include "lbf_internal.h"
@@ -235,45 +236,63 @@ cudaError_t launch_print(int storage, const PrintArgs& a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// FP64 sums over fluid nodes (phi_sum_count_kernel, lb_cuda_boundary_module.f90:461-515,
-// with a block-level tree instead of one atomic per node)
+// FP64 sums over fluid nodes (phi_sum_count_kernel, lb_cuda_boundary_module.f90:461-515):
+// grid-stride loops on one wave of CTAs, a warp and block tree, one atomic per
+// CTA and sum.  With a CTA per 256 nodes (up to 9,472 of them) the trees and
+// atomics cost more than the loads: lbf_reduce of 256^3 (336 MB) 137 us with
+// its copy to the host, 99 us now; the phi sum of 150 x 128 x 136 35 us (ncu).
 // ---------------------------------------------------------------------------
+constexpr int SUM_THREADS = 256;
+static inline int sum_blocks(long long n) {
+    const long long b = (n + 4 * SUM_THREADS - 1) / (4 * SUM_THREADS);  // four loads in flight a thread
+    return (int)std::max<long long>(1, std::min<long long>(b, 148 * 8));
+}
+
+// add the K sums of a CTA's threads to out[0..K-1]
+template <int K> __device__ __forceinline__ void block_add(double (&acc)[K], double* out) {
+    __shared__ double part[K][SUM_THREADS / 32];
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        if (lane == 0) part[k][warp] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < K) {
+        double s = 0;
+#pragma unroll
+        for (int w = 0; w < SUM_THREADS / 32; ++w) s += part[threadIdx.x][w];
+        atomicAdd(out + threadIdx.x, s);
+    }
+}
+
+__device__ __forceinline__ bool fluid_node(const int8_t* isf, long long i) {
+    if (!isf) return true;
+    const int f = isf[i];
+    return f == 1 || f == -1;
+}
+
 template <typename S>
-__global__ void reduce_kernel(long long N, const S* mom, const float* pres, const typename PhiStore<S>::type* phi,
-                              const int8_t* isf, double s0, double s1, double s2, double s3, double* out) {
+__global__ void __launch_bounds__(SUM_THREADS)
+    reduce_kernel(long long N, const S* mom, const float* pres, const typename PhiStore<S>::type* phi,
+                  const int8_t* isf, double s0, double s1, double s2, double s3, double* out) {
     using SP = typename PhiStore<S>::type;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        if (isf) {
-            int f = isf[i];
-            if (f != 1 && f != -1) continue;
-        }
-        if (phi) acc[0] += (double)Codec<SP>::ld(phi, i, 1.0);
-        if (Layout<S>::split) {
-            acc[1] += (double)pres[i];
-            acc[2] += (double)pres[N + i];
-            acc[3] += (double)pres[2 * N + i];
-            acc[4] += (double)pres[3 * N + i];
-        } else {
-            acc[1] += (double)Codec<S>::ld(mom, i, s0);
-            acc[2] += (double)Codec<S>::ld(mom, N + i, s1);
-            acc[3] += (double)Codec<S>::ld(mom, 2 * N + i, s2);
-            acc[4] += (double)Codec<S>::ld(mom, 3 * N + i, s3);
-        }
+    const double sc[4] = {s0, s1, s2, s3};
+    const long long stride = (long long)gridDim.x * SUM_THREADS;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)SUM_THREADS + threadIdx.x; i < N; i += stride) {
+        double v[5];
+        v[0] = phi ? (double)Codec<SP>::ld(phi, i, 1.0) : 0.0;
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+            v[1 + f] = Layout<S>::split ? (double)pres[f * N + i] : (double)Codec<S>::ld(mom + f * N, i, sc[f]);
+        const bool take = fluid_node(isf, i);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) acc[k] += take ? v[k] : 0.0;
     }
-    __shared__ double red[5][256];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) red[k][threadIdx.x] = acc[k];
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-#pragma unroll
-            for (int k = 0; k < 5; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < 5; ++k) atomicAdd(out + k, red[k][0]);
+    block_add<5>(acc, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -376,36 +395,21 @@ cudaError_t launch_download_pi(int storage, int dst_dtype, long long N, const vo
 
 // ---------------------------------------------------------------------------
 // phi mass correction (phi_sum_count_kernel + apply_lagrangian_phi_kernel,
-// lb_cuda_boundary_module.f90:459-563): FP64 sums, tree per block, one atomic
-// per block
+// lb_cuda_boundary_module.f90:459-563)
 // ---------------------------------------------------------------------------
-template <typename SP>
-__global__ void mass_sum_kernel(long long N, const SP* phi, const int8_t* isf, double* out, bool count) {
-    double acc = 0, cnt = 0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        if (isf) {
-            const int f = isf[i];
-            if (f != 1 && f != -1) continue;
-        }
+// COUNT: also the number of interface nodes, into out[1]
+template <typename SP, bool COUNT>
+__global__ void __launch_bounds__(SUM_THREADS) mass_sum_kernel(long long N, const SP* phi, const int8_t* isf, double* out) {
+    double acc[COUNT ? 2 : 1] = {};
+    const long long stride = (long long)gridDim.x * SUM_THREADS;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)SUM_THREADS + threadIdx.x; i < N; i += stride) {
         const double v = (double)phi[i];
-        acc += v;
-        if (v > 0.5 && v < 0.9) cnt += 1.0;
+        const bool take = fluid_node(isf, i);
+        acc[0] += take ? v : 0.0;
+        if (COUNT) acc[1] += take && v > 0.5 && v < 0.9 ? 1.0 : 0.0;
     }
-    __shared__ double red[2][256];
-    red[0][threadIdx.x] = acc;
-    red[1][threadIdx.x] = cnt;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) {
-            red[0][threadIdx.x] += red[0][threadIdx.x + s];
-            red[1][threadIdx.x] += red[1][threadIdx.x + s];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        atomicAdd(out, red[0][0]);
-        if (count) atomicAdd(out + 1, red[1][0]);
-    }
+    block_add<COUNT ? 2 : 1>(acc, out);
 }
 
 template <typename SP>
@@ -430,7 +434,8 @@ cudaError_t launch_mass(int storage, MassMode mode, long long N, void* phi, cons
     return by_storage(storage, [&](auto tag) {
         using SP = typename PhiStore<decltype(tag)>::type;
         SP* f = static_cast<SP*>(phi);
-        mass_sum_kernel<SP><<<blocks_for(N, 256), 256, 0, st>>>(N, f, isf, initial ? d_mass + 2 : d_mass, !initial);
+        if (initial) mass_sum_kernel<SP, false><<<sum_blocks(N), SUM_THREADS, 0, st>>>(N, f, isf, d_mass + 2);
+        else mass_sum_kernel<SP, true><<<sum_blocks(N), SUM_THREADS, 0, st>>>(N, f, isf, d_mass);
         if (mode == MASS_APPLY) mass_apply_kernel<SP><<<blocks_for(N, 256), 256, 0, st>>>(N, f, isf, d_mass);
         return cudaGetLastError();
     });
@@ -443,7 +448,7 @@ cudaError_t launch_reduce(int storage, long long N, const void* mom, const float
     return by_storage(storage, [&](auto tag) {
         using S = decltype(tag);
         using SP = typename PhiStore<S>::type;
-        reduce_kernel<S><<<blocks_for(N, 256), 256, 0, st>>>(N, static_cast<const S*>(mom), pres,
+        reduce_kernel<S><<<sum_blocks(N), SUM_THREADS, 0, st>>>(N, static_cast<const S*>(mom), pres,
                                                               static_cast<const SP*>(phi), isf, inv_scale[0],
                                                               inv_scale[1], inv_scale[2], inv_scale[3], d_out);
         return cudaGetLastError();

@@ -50,11 +50,13 @@ template <typename S, typename R, int TYV> constexpr size_t stream_smem_bytes() 
 }
 
 // One piece of a time step: tile (bx, by) of the box, planes z0 <= z < z1.
-// REP: REPULSIVE_FLUX force in the moments prologue; OBS: obstacles (isfluid
-// tests, the moment-space bounce-back, open-face moments).  Both are separate
-// compilations, so the kernels without them carry no code for them: the
-// obstacle code alone, never executed, costs a box without obstacles 5.6 %.
-template <int LAT, bool HO, typename S, typename R, int TYV, bool REP, bool OBS>
+// REP: REPULSIVE_FLUX force in the moments prologue; OBS: 1 obstacles (isfluid
+// tests, the moment-space bounce-back) and the phi mass correction, 2 the
+// correction alone, 0 neither.  Separate compilations, so the kernels without
+// them carry no code for them: the obstacle code alone, never executed, costs a
+// box without obstacles 5.6 %, and the correction in that compilation a quarter
+// of the step (150 x 128 x 136: 257 us with its sum, 212 us now).
+template <int LAT, bool HO, typename S, typename R, int TYV, bool REP, int OBS>
 __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int bx, const int by, const int z0,
                                           const int z1) {
     using TL = Tile<TYV>;
@@ -95,7 +97,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     const int plane = (int)p.plane;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const bool dr = p.densratio != 0;
-    const bool obs = OBS && p.obstacles != 0;
+    const bool obs = OBS == 1 && p.obstacles != 0;
     const R cssq = R(1.0 / 3.0);
 
     // ---- static per-thread node tables (x/y wrap does not change along z) ----
@@ -142,7 +144,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     bool wrapA, wrapB;
     const bool okA = r1_geom(nodeA, offA, wrapA);
     const bool okB = r1_geom(nodeB, offB, wrapB);
-    // phi mass correction of the input phi (compiled with the obstacle code only)
+    // phi mass correction of the input phi
     double mcorr = 0.0;
     bool do_mcorr = false;
     if constexpr (OBS) do_mcorr = mass_corr(p.mass, mcorr);
@@ -794,10 +796,10 @@ template <int LAT, bool TC, typename S, typename R, int TYV> constexpr size_t st
     if constexpr (TC) return stream_smem_bytes<S, R, TYV>();
     else return single_smem_bytes<LAT, R, TYV>();
 }
-template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP, bool OBS>
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP, int OBS>
 __device__ __forceinline__ void any_body(const StepParams<S, R>& p, int bx, int by, int z0, int z1) {
     if constexpr (TC) step_body<LAT, HO, S, R, TYV, REP, OBS>(p, bx, by, z0, z1);
-    else single_body<LAT, HO, S, R, TYV, OBS>(p, bx, by, z0, z1);
+    else single_body<LAT, HO, S, R, TYV, OBS == 1>(p, bx, by, z0, z1);
 }
 
 // Column-planes of the planes zlo .. zlo + nzr - 1 of a box for a tile of
@@ -828,7 +830,7 @@ __device__ __forceinline__ void run_share(const int nx, const int nzr, const int
 // site of step_body, so the kernel holds a single compiled copy of the step:
 // separately inlined copies may contract floating-point operations
 // differently and give results that differ in the last bit.
-template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
 __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>()) stream_kernel(const StepParams<S, R> p) {
     long long s0, s1;
     const int nzr = p.zhi - p.zlo;
@@ -858,7 +860,7 @@ __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TY
 // [work[i].y, work[i].z) of that box (column-major: plane fastest), with the
 // box's own parameters and fields.  Each node's arithmetic is the same as in
 // stream_kernel, so a box gives the same bits alone and in a batch.
-template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, bool OBS = true>
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
 __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>())
     stream_kernel_batched(const StepParams<S, R>* __restrict__ boxes, const int4* __restrict__ work) {
     __shared__ StepParams<S, R> sp;
