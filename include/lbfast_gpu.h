@@ -377,7 +377,8 @@ int lbf_server_submit(lbf_server* s, const lbf_params* p, const int8_t* isfluid,
 /* Admits queued solves that fit, advances the resident ones by up to
  * max_chunks chunks (each ends with a device synchronisation), and retires
  * finished solves (their fields are copied to host memory and their device
- * memory is released, which may admit more).  Returns after max_chunks chunks
+ * memory goes back to the server's pool, which may admit more; an idle server
+ * keeps at most 256 MB of it).  Returns after max_chunks chunks
  * or when nothing is resident; *active and *queued (either may be NULL) give
  * the counts on return. */
 int lbf_server_run(lbf_server* s, int max_chunks, int* active, int* queued);
@@ -385,7 +386,8 @@ int lbf_server_poll(lbf_server* s, long long id, lbf_solve_info* info);
 /* Copies a finished solve's mom10 and phi (either may be NULL) in the dtype it
  * was submitted with and forgets it; LBF_E_STATE until it is done. */
 int lbf_server_fetch(lbf_server* s, long long id, void* mom10, void* phi);
-/* Drops a queued or resident solve; its device memory is released at once. */
+/* Drops a queued or resident solve; its device memory goes back to the
+ * server's pool at once. */
 int lbf_server_cancel(lbf_server* s, long long id);
 /* Device bytes a solve of these parameters holds while resident. */
 long long lbf_server_solve_bytes(const lbf_params* p);

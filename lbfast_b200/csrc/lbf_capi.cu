@@ -61,12 +61,30 @@ void record_error(const char* msg) { g_last_error = msg; }
 
 namespace {
 
+template <typename T> bool dev_alloc(lbf_handle* h, T*& p, size_t bytes) {
+    void* q = nullptr;
+    cudaError_t e = h->pool ? cudaMallocFromPoolAsync(&q, bytes, h->pool, h->stream) : cudaMalloc(&q, bytes);
+    if (e != cudaSuccess && h->pool) {
+        // no block of the pool fits: give its unused ones back and try again
+        cudaGetLastError();
+        cudaStreamSynchronize(h->stream);
+        cudaMemPoolTrimTo(h->pool, 0);
+        e = cudaMallocFromPoolAsync(&q, bytes, h->pool, h->stream);
+    }
+    p = static_cast<T*>(q);
+    return e == cudaSuccess;
+}
+template <typename T> void dev_free(lbf_handle* h, T*& p) {
+    if (p && h->pool) cudaFreeAsync(p, h->stream);
+    else cudaFree(p);
+    p = nullptr;
+}
+
 int ensure_staging(lbf_handle* h, size_t bytes) {
     if (h->staging_bytes >= bytes) return LBF_OK;
-    if (h->staging) cudaFree(h->staging);
-    h->staging = nullptr;
+    dev_free(h, h->staging);
     h->staging_bytes = 0;
-    if (cudaMalloc(&h->staging, bytes) != cudaSuccess)
+    if (!dev_alloc(h, h->staging, bytes))
         return fail(LBF_E_NOMEM, "device staging allocation of %zu bytes failed", bytes);
     h->staging_bytes = bytes;
     return LBF_OK;
@@ -84,13 +102,13 @@ template <typename T> int replace_table(T*& t, const std::vector<T>& v) {
 
 void free_all(lbf_handle* h) {
     for (int b = 0; b < 2; ++b) {
-        cudaFree(h->mom[b]);
-        cudaFree(h->uold[b]);
-        cudaFree(h->phi[b]);
-        cudaFree(h->pres[b]);
+        dev_free(h, h->mom[b]);
+        dev_free(h, h->uold[b]);
+        dev_free(h, h->phi[b]);
+        dev_free(h, h->pres[b]);
         cudaFree(h->wetW[b]);
     }
-    cudaFree(h->isf);
+    dev_free(h, h->isf);
     cudaFree(h->link_rows);
     cudaFree(h->links);
     cudaFree(h->wet_s);
@@ -98,14 +116,14 @@ void free_all(lbf_handle* h) {
     cudaFree(h->wet_flag);
     cudaFree(h->wet_wn);
     cudaFree(h->wet_shift);
-    cudaFree(h->d_err);
-    cudaFree(h->d_red);
-    cudaFree(h->d_mass);
+    dev_free(h, h->d_err);
+    dev_free(h, h->d_red);
+    dev_free(h, h->d_mass);
     cudaFree(h->wall_nodes);
     cudaFree(h->wall_links);
-    cudaFree(h->d_rnrm);
-    cudaFree(h->d_rep);
-    cudaFree(h->staging);
+    dev_free(h, h->d_rnrm);
+    dev_free(h, h->d_rep);
+    dev_free(h, h->staging);
     if (h->xstream) cudaStreamDestroy(h->xstream);
     if (h->ev_done) cudaEventDestroy(h->ev_done);
     if (h->ev_copied) cudaEventDestroy(h->ev_copied);
@@ -363,7 +381,11 @@ int lbf_last_error(char* buf, size_t n) {
     return LBF_OK;
 }
 
-int lbf_create(const lbf_params* p, lbf_handle** out) {
+int lbf_create(const lbf_params* p, lbf_handle** out) { return lbf::handle_create(p, nullptr, nullptr, out); }
+
+}  // extern "C"
+
+int lbf::handle_create(const lbf_params* p, cudaMemPool_t pool, cudaStream_t st, lbf_handle** out) {
     if (!p || !out) return fail(LBF_E_ARG, "lbf_create: null argument");
     *out = nullptr;
     if (p->lx < 1 || p->ly < 1 || p->lz < 1) return fail(LBF_E_ARG, "box must be at least 1^3");
@@ -430,22 +452,24 @@ int lbf_create(const lbf_params* p, lbf_handle** out) {
     }
     // > 0: z segments; < 0: columns split at plane -zseg; 0: persistent schedule
     h->zseg = p->zseg > 0 ? std::min(p->zseg, p->lz) : (p->zseg < 0 ? std::max(p->zseg, -p->lz) : 0);
+    h->pool = pool;
+    h->stream = st;
     bool ok = true;
     for (int b = 0; b < 2 && ok; ++b) {
         // 16-bit storage: Pi - u u (6 fields) in 16 bits, P, u, v, w in FP32 (pres)
-        ok = ok && cudaMalloc(&h->mom[b], (is_half(h->storage) ? 6 : 10) * h->N * h->esz) == cudaSuccess;
-        ok = ok && cudaMalloc(&h->uold[b], 3 * h->N * h->esz) == cudaSuccess;
-        if (h->tc) ok = ok && cudaMalloc(&h->phi[b], h->N * h->psz) == cudaSuccess;
-        if (is_half(h->storage)) ok = ok && cudaMalloc(&h->pres[b], 4 * h->N * sizeof(float)) == cudaSuccess;
+        ok = ok && dev_alloc(h, h->mom[b], (is_half(h->storage) ? 6 : 10) * h->N * h->esz);
+        ok = ok && dev_alloc(h, h->uold[b], 3 * h->N * h->esz);
+        if (h->tc) ok = ok && dev_alloc(h, h->phi[b], h->N * h->psz);
+        if (is_half(h->storage)) ok = ok && dev_alloc(h, h->pres[b], 4 * h->N * sizeof(float));
     }
-    if (ok && h->obs) ok = cudaMalloc(&h->isf, h->N) == cudaSuccess;
-    if (ok) ok = cudaMalloc(&h->d_err, sizeof(int)) == cudaSuccess;
-    if (ok) ok = cudaMalloc(&h->d_red, 5 * sizeof(double)) == cudaSuccess;
-    if (ok && p->phi_correction) ok = cudaMalloc(&h->d_mass, 4 * sizeof(double)) == cudaSuccess;
+    if (ok && h->obs) ok = dev_alloc(h, h->isf, h->N);
+    if (ok) ok = dev_alloc(h, h->d_err, sizeof(int));
+    if (ok) ok = dev_alloc(h, h->d_red, 5 * sizeof(double));
+    if (ok && p->phi_correction) ok = dev_alloc(h, h->d_mass, 4 * sizeof(double));
     if (p->openbc) h->obc_open = (p->pbc_x ? 0 : 1) | (p->pbc_y ? 0 : 2) | (p->pbc_z ? 0 : 4);
     if (ok && p->repulsive_flux) {
-        ok = cudaMalloc(&h->d_rnrm, 3 * h->N * sizeof(double)) == cudaSuccess;
-        if (ok) ok = cudaMalloc(&h->d_rep, 3 * h->N * (p->storage == LBF_STORE_F64 ? 8 : 4)) == cudaSuccess;
+        ok = dev_alloc(h, h->d_rnrm, 3 * h->N * sizeof(double));
+        if (ok) ok = dev_alloc(h, h->d_rep, 3 * h->N * (p->storage == LBF_STORE_F64 ? 8 : 4));
     }
     if (!ok) {
         cudaGetLastError();
@@ -454,12 +478,14 @@ int lbf_create(const lbf_params* p, lbf_handle** out) {
         delete h;
         return fail(LBF_E_NOMEM, "device allocation of %.3f GB failed", need / 1e9);
     }
-    cudaMemset(h->d_err, 0, sizeof(int));
-    if (h->obs) cudaMemset(h->isf, 1, h->N);
-    if (h->d_mass) cudaMemset(h->d_mass, 0, 4 * sizeof(double));
+    cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
+    if (h->obs) cudaMemsetAsync(h->isf, 1, h->N, h->stream);
+    if (h->d_mass) cudaMemsetAsync(h->d_mass, 0, 4 * sizeof(double), h->stream);
     *out = h;
     return LBF_OK;
 }
+
+extern "C" {
 
 int lbf_destroy(lbf_handle* h) {
     if (!h) return fail(LBF_E_ARG, "lbf_destroy: null handle");
@@ -1383,9 +1409,7 @@ int handle_post_step(lbf_handle* h) {
 bool handle_steady(const lbf_handle* h) { return !(h->tc && h->obs && h->nwet > 0) || h->wet_pending >= 0; }
 
 void handle_release_staging(lbf_handle* h) {
-    if (!h->staging) return;
-    cudaFree(h->staging);
-    h->staging = nullptr;
+    dev_free(h, h->staging);
     h->staging_bytes = 0;
 }
 

@@ -40,6 +40,9 @@ struct lbf_handle {
     int wet_pending_target = -1;  // phi buffer they belong to
     double cot_theta = 0;
     cudaStream_t stream = nullptr;
+    // the state's and the staging buffer's allocator: a pool of the server that
+    // owns the handle (stream-ordered on `stream`), or cudaMalloc when null
+    cudaMemPool_t pool = nullptr;
     int* d_err = nullptr;
     double* d_red = nullptr;
     void* staging = nullptr;
@@ -74,6 +77,8 @@ constexpr int SLAB_HALO = 3;
 }  // namespace lbf
 
 namespace lbf {
+// lbf_create with the device memory of `pool` on stream st (null: lbf_create)
+int handle_create(const lbf_params* p, cudaMemPool_t pool, cudaStream_t st, lbf_handle** out);
 // integrator pre-loop work (wetting) of a freshly filled handle
 int handle_prime(lbf_handle* h);
 // launch arguments of the next step of h (its current time level)
