@@ -216,17 +216,18 @@ int autotune(lbf_handle* h) {
             // exactly but staggers neighbours in z.
             const int za = auto_zseg(h->nx, h->ny, h->nz, ty), lo = std::min(h->nz, 8);
             std::vector<int> all = {0, za, std::max(lo, za / 2), std::min(h->nz, 2 * za), h->nz};
-            // small boxes, whose columns in segments of 8 planes leave SMs
-            // empty: segments that fill one wave and two waves of CTA slots.
-            // The pipeline fill of a segment costs 3-4 planes' time, an empty
-            // SM all of it: 32^3 with two components (2 columns) steps in
-            // 22.6 us in one-plane segments against 49.2 us in segments of 8,
-            // 64^3 (8 columns) in 34.9 us in segments of 4
+            // segments that fill one wave and two waves of CTA slots.  A
+            // segment's pipeline fill costs 3-4 planes' time, an empty SM all of
+            // it: 32^3 with two components (2 columns) steps in 22.6 us in
+            // one-plane segments against 49.2 us in segments of 8, 64^3 (8
+            // columns) in 34.9 us in segments of 4, FP64 96 x 88 x 104 (33
+            // columns) in 127 us in four segments a column against 148 us in
+            // the best of the others
             const long long cols = (long long)((h->nx + 31) / 32) * ((h->ny + ty - 1) / ty);
             const int nzr = h->slab ? h->nzs : h->nz;
             const long long slots = lbf::resident_slots((ty == 8 && h->storage != LBF_STORE_F64) ? 2 : 1);
             for (long long w = slots; w <= 2 * slots; w += slots)
-                if (cols < w && (cols * nzr + w - 1) / w < 8) all.push_back((int)((cols * nzr + w - 1) / w));
+                if (cols < w) all.push_back((int)((nzr + w / cols - 1) / (w / cols)));
             // split columns (negative: the split plane)
             for (int L : split_planes(h->nx, h->ny, h->slab ? h->nzs : h->nz, ty, h->storage)) all.push_back(-L);
             for (int z : all)
