@@ -2,6 +2,7 @@
 // storage type by lbf_inst_<storage>.cu so the instantiations compile in
 // parallel.
 #pragma once
+#include "lbf_chain.cuh"
 #include "lbf_internal.h"
 #include "lbf_stream_kernel.cuh"
 
@@ -62,13 +63,12 @@ cudaError_t launch_stream(const StepArgs& a, cudaStream_t st) {
     if (a.zseg < 0) {
         // split columns: a head and a tail segment per column
         const long long ncols = (long long)((a.nx + TX - 1) / TX) * ((a.ny + TYV - 1) / TYV);
-        stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<(unsigned)(2 * ncols), step_threads<TC, TYV>(), smem, st>>>(p);
-        return cudaGetLastError();
+        return launch_chained(stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS>, dim3((unsigned)(2 * ncols)),
+                              step_threads<TC, TYV>(), smem, st, p);
     }
     if (a.zseg > 0) {
         dim3 grid((a.nx + TX - 1) / TX, (a.ny + TYV - 1) / TYV, (nzr + a.zseg - 1) / a.zseg);
-        stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<grid, step_threads<TC, TYV>(), smem, st>>>(p);
-        return cudaGetLastError();
+        return launch_chained(stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS>, grid, step_threads<TC, TYV>(), smem, st, p);
     }
     static int resident = 0;  // CTAs per SM at this shared-memory size
     if (!resident) {
@@ -79,8 +79,7 @@ cudaError_t launch_stream(const StepArgs& a, cudaStream_t st) {
     }
     const long long W = (long long)((a.nx + TX - 1) / TX) * ((a.ny + TYV - 1) / TYV) * nzr;
     const int grid = persistent_grid(W, resident);
-    stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS><<<grid, step_threads<TC, TYV>(), smem, st>>>(p);
-    return cudaGetLastError();
+    return launch_chained(stream_kernel<LAT, HO, TC, S, R, TYV, REP, OBS>, dim3(grid), step_threads<TC, TYV>(), smem, st, p);
 }
 
 // One launch advancing many boxes of one kernel class: d_boxes holds one
@@ -97,9 +96,8 @@ cudaError_t launch_stream_batched(const void* d_boxes, const int4* d_work, int n
         attr_set = true;
     }
     if (nwork <= 0) return cudaSuccess;
-    stream_kernel_batched<LAT, HO, TC, S, R, TYV, REP, OBS>
-        <<<nwork, step_threads<TC, TYV>(), smem, st>>>(static_cast<const StepParams<S, R>*>(d_boxes), d_work);
-    return cudaGetLastError();
+    return launch_chained(stream_kernel_batched<LAT, HO, TC, S, R, TYV, REP, OBS>, dim3(nwork), step_threads<TC, TYV>(), smem,
+                          st, static_cast<const StepParams<S, R>*>(d_boxes), d_work);
 }
 
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1> int batched_resident() {

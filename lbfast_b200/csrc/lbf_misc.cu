@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "lbf_chain.cuh"
 #include "lbf_internal.h"
 #include "lbf_stream.cuh"
 
@@ -50,6 +51,7 @@ static inline int blocks_for(long long n, int bs) {
 // ---------------------------------------------------------------------------
 template <typename SP, typename R>
 __global__ void wetting_kernel(const WetArgs a) {
+    chain_begin();
     using CP = Codec<SP>;
     const SP* pin = static_cast<const SP*>(a.pin);
     SP* wout = static_cast<SP*>(a.wout);
@@ -112,8 +114,7 @@ cudaError_t launch_wetting(int storage, const WetArgs& a, cudaStream_t st) {
         using S = decltype(tag);
         using SP = typename PhiStore<S>::type;
         using R = typename Arith<S>::R;
-        wetting_kernel<SP, R><<<blocks_for(a.n, 256), 256, 0, st>>>(a);
-        return cudaGetLastError();
+        return launch_chained(wetting_kernel<SP, R>, dim3(blocks_for(a.n, 256)), 256, 0, st, a);
     });
 }
 

@@ -9,6 +9,7 @@
 // FP64, as the reference's (real(kind=db)).
 #include <type_traits>
 
+#include "lbf_chain.cuh"
 #include "lbf_internal.h"
 #include "lbf_stream.cuh"
 
@@ -78,6 +79,7 @@ __device__ __forceinline__ void tile_origin(const RepulsiveArgs& a, int& X0, int
 // only ones that the search compares (a partner passes the same threshold as
 // the node itself), so the others' slots keep whatever they hold.
 template <typename SP> __global__ void __launch_bounds__(RTHREADS, 3) rep_normals_kernel(const RepulsiveArgs a) {
+    chain_begin();
     const long long N = (long long)a.nx * a.ny * a.nz;
     const SearchPhi<SP> PH(a);
     int X0, Y0, Z0;
@@ -146,6 +148,7 @@ template <typename SP, typename R> __global__ void __launch_bounds__(RTHREADS) r
     const long long N = (long long)a.nx * a.ny * a.nz;
     R* out = static_cast<R*>(a.force);
     const double eps = 1.0e-9;
+    chain_begin();
     const SearchPhi<SP> PH(a);
     int X0, Y0, Z0;
     tile_origin(a, X0, Y0, Z0);
@@ -318,9 +321,9 @@ cudaError_t launch_repulsive(int storage, const RepulsiveArgs& a, cudaStream_t s
         using S = decltype(tag);
         using SP = typename PhiStore<S>::type;
         using R = typename std::conditional<sizeof(S) == 8, double, float>::type;
-        rep_normals_kernel<SP><<<(unsigned)tiles, RTHREADS, 0, st>>>(a);
-        rep_force_kernel<SP, R><<<(unsigned)tiles, RTHREADS, 0, st>>>(a);
-        return cudaGetLastError();
+        const cudaError_t e = launch_chained(rep_normals_kernel<SP>, dim3((unsigned)tiles), RTHREADS, 0, st, a);
+        if (e != cudaSuccess) return e;
+        return launch_chained(rep_force_kernel<SP, R>, dim3((unsigned)tiles), RTHREADS, 0, st, a);
     });
 }
 

@@ -13,6 +13,7 @@
 //            pulls the populations of plane q and plane q-1 is written.  The
 //            copy completes behind this phase.
 #pragma once
+#include "lbf_chain.cuh"
 #include "lbf_node.cuh"
 #include "lbf_single_kernel.cuh"
 
@@ -832,6 +833,7 @@ __device__ __forceinline__ void run_share(const int nx, const int nzr, const int
 // differently and give results that differ in the last bit.
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
 __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>()) stream_kernel(const StepParams<S, R> p) {
+    chain_begin();
     long long s0, s1;
     const int nzr = p.zhi - p.zlo;
     if (p.zseg < 0) {
@@ -864,6 +866,7 @@ template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP =
 __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>())
     stream_kernel_batched(const StepParams<S, R>* __restrict__ boxes, const int4* __restrict__ work) {
     __shared__ StepParams<S, R> sp;
+    chain_begin();
     const int4 w = work[blockIdx.x];
     if (threadIdx.x == 0) sp = boxes[w.x];
     __syncthreads();

@@ -10,6 +10,7 @@
 // carries no code for them.
 #include <type_traits>
 
+#include "lbf_chain.cuh"
 #include "lbf_internal.h"
 #include "lbf_node.cuh"
 
@@ -346,6 +347,7 @@ template <typename S, int LAT, bool HO>
 __global__ void __launch_bounds__(WALL_THREADS) wall_kernel(const BoundaryArgs a) {
     const long long plane = (long long)a.nx * a.ny, N = plane * a.nz;
     const double cssq = 1.0 / 3.0;
+    chain_begin();
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= a.nnodes) return;
     const long long g = a.nodes[t];
@@ -470,11 +472,10 @@ cudaError_t launch_walls(int storage, const BoundaryArgs& a, cudaStream_t st) {
     const unsigned grid = (unsigned)((a.nnodes + WALL_THREADS - 1) / WALL_THREADS);
     return by_storage(storage, [&](auto tag) {
         using S = decltype(tag);
-        if (a.lattice == 27 && a.highorder) wall_kernel<S, 27, true><<<grid, WALL_THREADS, 0, st>>>(a);
-        else if (a.lattice == 27) wall_kernel<S, 27, false><<<grid, WALL_THREADS, 0, st>>>(a);
-        else if (a.lattice == 19) wall_kernel<S, 19, false><<<grid, WALL_THREADS, 0, st>>>(a);
-        else wall_kernel<S, 15, false><<<grid, WALL_THREADS, 0, st>>>(a);
-        return cudaGetLastError();
+        if (a.lattice == 27 && a.highorder) return launch_chained(wall_kernel<S, 27, true>, dim3(grid), WALL_THREADS, 0, st, a);
+        if (a.lattice == 27) return launch_chained(wall_kernel<S, 27, false>, dim3(grid), WALL_THREADS, 0, st, a);
+        if (a.lattice == 19) return launch_chained(wall_kernel<S, 19, false>, dim3(grid), WALL_THREADS, 0, st, a);
+        return launch_chained(wall_kernel<S, 15, false>, dim3(grid), WALL_THREADS, 0, st, a);
     });
 }
 
