@@ -65,10 +65,37 @@ __device__ __forceinline__ void d1q3n2(T m0, T m1, T m2n, T& vm, T& v0, T& vp) {
 
 // HIGHORDER coefficients, rows 10..26 of the reference
 // (lb_cuda_fused_module.f90:667-703): each the equilibrium monomial + om1 x
-// its non-equilibrium projection, with the factors that rows share taken out:
-// about 90 operations, 160 as the reference writes them out (5.7 % fewer warp
-// instructions in the two-component FP32 step, whose time stays within 1 %: it
-// waits on latency).
+// its non-equilibrium projection.  Two forms.  `ho_rows` takes out the factors
+// that rows share: about 90 operations against 160, but longer chains of them.
+// The one-component step, which waits on issue, is faster with it (200 x 184 x
+// 168: 276 -> 266 us), and so is the two-component one with obstacles, which
+// sits at the register limit (512 x 256 x 256 channel: 2.74 -> 2.43 ms); the
+// plain two-component one, which waits on latency, is not (256^3: 917 -> 928 us
+// with 5.7 % fewer instructions) and takes `ho_rows_wide`.
+template <typename R>
+__device__ __forceinline__ void ho_rows_wide(R (&M)[3][3][3], const R u, const R v, const R w, const R om1, const R X,
+                                             const R Y, const R Z, const R XY, const R XZ, const R YZ) {
+    const R u2 = u * u, v2 = v * v, w2 = w * w;
+    M[2][1][0] = u2 * v + om1 * (R(2) * XY * u + X * v);
+    M[2][0][1] = u2 * w + om1 * (R(2) * XZ * u + X * w);
+    M[1][2][0] = u * v2 + om1 * (Y * u + R(2) * XY * v);
+    M[1][0][2] = u * w2 + om1 * (Z * u + R(2) * XZ * w);
+    M[0][1][2] = v * w2 + om1 * (Z * v + R(2) * YZ * w);
+    M[0][2][1] = v2 * w + om1 * (R(2) * YZ * v + Y * w);
+    M[1][1][1] = u * v * w + om1 * (YZ * u + XZ * v + XY * w);
+    M[2][2][0] = u2 * v2 + om1 * (Y * u2 + R(2) * v * (R(3) * XY * u + X * v));
+    M[2][0][2] = u2 * w2 + om1 * (Z * u2 + R(2) * w * (R(3) * XZ * u + X * w));
+    M[0][2][2] = v2 * w2 + om1 * (Z * v2 + R(2) * w * (R(3) * YZ * v + Y * w));
+    M[1][1][2] = u * v * w2 + om1 * (Z * u * v + w * (R(3) * YZ * u + R(3) * XZ * v + R(2) * XY * w));
+    M[1][2][1] = u * v2 * w + om1 * (R(2) * YZ * u * v + XZ * v2 + R(2) * Y * u * w + R(4) * XY * v * w);
+    M[2][1][1] = u2 * v * w + om1 * (YZ * u2 + R(2) * XZ * u * v + R(4) * XY * u * w + R(2) * X * v * w);
+    M[2][1][2] = u2 * v * w2 + om1 * (Z * u2 * v + R(3) * w * (YZ * u2 + R(2) * XZ * u * v + R(2) * XY * u * w + X * v * w));
+    M[2][2][1] = u2 * v2 * w + om1 * (R(2) * u * v * (YZ * u + XZ * v) + R(2) * Y * u2 * w +
+                                      v * (R(10) * XY * u + R(3) * X * v) * w);
+    M[1][2][2] = u * v2 * w2 + om1 * (Z * u * v2 + R(3) * w * (R(2) * YZ * u * v + XZ * v2 + Y * u * w + R(2) * XY * v * w));
+    M[2][2][2] = u2 * v2 * w2 + om1 * (Z * u2 * v2 + w * (R(6) * u * v * (YZ * u + XZ * v) + R(3) * Y * u2 * w +
+                                                          R(2) * v * (R(7) * XY * u + R(2) * X * v) * w));
+}
 template <typename R>
 __device__ __forceinline__ void ho_rows(R (&M)[3][3][3], const R u, const R v, const R w, const R om1, const R Xn,
                                         const R Yn, const R Zn, const R XYn, const R XZn, const R YZn) {

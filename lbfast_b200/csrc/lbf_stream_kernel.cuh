@@ -678,7 +678,8 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                     M[2][0][0] = mxx; M[0][2][0] = myy; M[0][0][2] = mzz;
                     M[1][1][0] = mxy; M[1][0][1] = mxz; M[0][1][1] = myz;
                     if constexpr (HO) {
-                        ho_rows<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
+                        if constexpr (OBS != 0) ho_rows<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
+                        else ho_rows_wide<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
                     } else {
                         M[2][1][0] = M[2][0][1] = M[1][2][0] = M[1][0][2] = M[0][1][2] = M[0][2][1] = M[1][1][1] = R(0);
                         M[2][2][0] = M[2][0][2] = M[0][2][2] = M[1][1][2] = M[1][2][1] = M[2][1][1] = R(0);
