@@ -141,9 +141,9 @@ struct lbf_server {
     // solve takes over the memory of the ones before it.  With cudaMalloc and
     // cudaFree a 64^3 solve spent 4.6 ms on its dozen buffers, more than on its
     // steps (12 solves of 32^3-64^3, 64 steps each, submitted and fetched: 84 ms,
-    // 55 ms now).  Unused
-    // blocks above the memory budget are given back at each admission, all but
-    // POOL_KEEP when the server is idle, the rest when it is destroyed.
+    // 55 ms now).  Unused blocks above the memory budget are given back at each
+    // admission, all but POOL_KEEP when the server is idle, the rest when it is
+    // destroyed.
     cudaMemPool_t pool = nullptr;
     long long next_id = 1;
     std::map<long long, std::unique_ptr<Solve>> solves;
