@@ -16,6 +16,16 @@ template <typename R> __device__ __forceinline__ R sqrt_a(R x);
 template <> __device__ __forceinline__ float sqrt_a<float>(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 template <> __device__ __forceinline__ double sqrt_a<double>(double x) { return sqrt(x); }
 
+// A product that several terms read, rounded on its own: the compiler may
+// contract a plain a * b into some of the sums it enters and not into others,
+// and which ones depends on the code around it.  The one-component step is two
+// compilations of each lattice (with and without HIGHORDER) in four storage
+// types; with the products of its collision left to the compiler, D3Q27 runs in
+// bfloat16 moved by 4e-4 of the result between one form of the kernel and the next.
+template <typename R> __device__ __forceinline__ R mul_rn(R a, R b);
+template <> __device__ __forceinline__ float mul_rn<float>(float a, float b) { return __fmul_rn(a, b); }
+template <> __device__ __forceinline__ double mul_rn<double>(double a, double b) { return __dmul_rn(a, b); }
+
 // Smagorinsky constant of the reference: the single-precision product 0.053 * 18.0
 constexpr double SMAG_C = (double)(0.053f * 18.0f);
 
@@ -65,13 +75,13 @@ __device__ __forceinline__ void d1q3n2(T m0, T m1, T m2n, T& vm, T& v0, T& vp) {
 
 // HIGHORDER coefficients, rows 10..26 of the reference
 // (lb_cuda_fused_module.f90:667-703): each the equilibrium monomial + om1 x
-// its non-equilibrium projection.  Two forms.  `ho_rows` takes out the factors
-// that rows share: about 90 operations against 160, but longer chains of them.
-// The one-component step, which waits on issue, is faster with it (200 x 184 x
-// 168: 276 -> 266 us), and so is the two-component one with obstacles, which
-// sits at the register limit (512 x 256 x 256 channel: 2.74 -> 2.43 ms); the
-// plain two-component one, which waits on latency, is not (256^3: 917 -> 928 us
-// with 5.7 % fewer instructions) and takes `ho_rows_wide`.
+// its non-equilibrium projection.  Two forms.  `ho_rows_wide` is the
+// reference's own.  `ho_rows` takes out the factors that rows share: about 90
+// operations against 160, but longer chains of them, and other roundings.  The
+// two-component step with obstacles, which sits at the register limit, takes it
+// (512 x 256 x 256 channel: 2.74 -> 2.43 ms); the plain two-component one, which
+// waits on latency, is slower with it (256^3: 917 -> 928 us with 5.7 % fewer
+// instructions).
 template <typename R>
 __device__ __forceinline__ void ho_rows_wide(R (&M)[3][3][3], const R u, const R v, const R w, const R om1, const R X,
                                              const R Y, const R Z, const R XY, const R XZ, const R YZ) {
@@ -220,39 +230,45 @@ __device__ __forceinline__ void ring_row_pops27(const R (&M)[3][3][3], const R d
     }
 }
 
-// Second-order populations of D3Q19 / D3Q15 (by D3Q27 link), the links in
-// opposite pairs: the even part of the expansion +- its odd part.  The factor
-// 3 of the odd part goes to the moments, not to the weight: 3 w rounds by up to
-// 3e-8 in FP32, w by less than 1e-8, and either scales the momentum in every
-// step.
+// Second-order populations of D3Q19 / D3Q15 (by D3Q27 link):
+// w ((base + 3 m.c) + 4.5 c c:m_diagonal + 9 c c:m_off-diagonal), the terms
+// added in this order.  Opposite links differ in the sign of m.c alone and go
+// as a pair.  (The even terms first, once for both links, are two operations
+// less a pair; but the order of the sums decides which 16-bit stored values
+// round up, and that one moved bfloat16 runs by 1.6e-4 of the result.)
 template <int LAT, typename R>
 __device__ __forceinline__ void low_order_pops(const R m0, const R mx, const R my, const R mz, const R mxx, const R myy,
                                                const R mzz, const R mxy, const R mxz, const R myz, R (&fpop)[27]) {
+    using P = PK<R>;
     const R base = m0 - R(1.5) * (mxx + myy + mzz);
-    const R m1[3] = {R(3) * mx, R(3) * my, R(3) * mz}, m2[3] = {mxx, myy, mzz};
+    const R m1[3] = {mx, my, mz}, m2[3] = {mxx, myy, mzz}, mc[3] = {mxy, mxz, myz};
     fpop[0] = R(WL<LAT>(0)) * base;
 #pragma unroll
     for (int l = 1; l < 27; l += 2) {
         if (!IN<LAT>(l)) continue;
-        const int c[3] = {EX(l), EY(l), EZ(l)};
-        R odd = R(0), diag = R(0);
-        bool first = true;  // the sums start with their first term, not with 0 + it
+        const int c[3] = {EX(l), EY(l), EZ(l)}, cc[3] = {c[0] * c[1], c[0] * c[2], c[1] * c[2]};
+        R odd = R(0), diag = R(0), off = R(0);
+        bool first = true, first_off = true;  // the sums start with their first term, not with 0 + it
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            if (!c[d]) continue;
-            const R m = c[d] > 0 ? m1[d] : -m1[d];
-            odd = first ? m : odd + m;
-            diag = first ? m2[d] : diag + m2[d];
-            first = false;
+            if (c[d]) {
+                const R m = c[d] > 0 ? m1[d] : -m1[d];
+                odd = first ? m : odd + m;
+                diag = first ? m2[d] : diag + m2[d];
+                first = false;
+            }
+            if (cc[d]) {
+                const R m = cc[d] > 0 ? mc[d] : -mc[d];
+                off = first_off ? m : off + m;
+                first_off = false;
+            }
         }
-        R even = fmaf_t(R(4.5), diag, base);
-        if (c[0] * c[1]) even = fmaf_t(R(9 * c[0] * c[1]), mxy, even);
-        if (c[0] * c[2]) even = fmaf_t(R(9 * c[0] * c[2]), mxz, even);
-        if (c[1] * c[2]) even = fmaf_t(R(9 * c[1] * c[2]), myz, even);
-        const R w = R(WL<LAT>(l));
-        const R we = w * even;
-        fpop[l] = fmaf_t(w, odd, we);
-        fpop[l + 1] = fmaf_t(-w, odd, we);
+        typename P::T f = P::fma(P::mk(R(3), R(-3)), P::mk(odd, odd), P::mk(base, base));
+        f = P::fma(P::mk(R(4.5), R(4.5)), P::mk(diag, diag), f);
+        if (!first_off) f = P::fma(P::mk(R(9), R(9)), P::mk(off, off), f);
+        f = P::mul(P::mk(R(WL<LAT>(l)), R(WL<LAT>(l))), f);
+        fpop[l] = f.x;
+        fpop[l + 1] = f.y;
     }
 }
 

@@ -10,11 +10,16 @@
 //  * every node's fields, the ring's too, are loaded one plane ahead;
 //  * links that the lattice lacks are neither stored nor summed, and D3Q19 /
 //    D3Q15 populations are built in opposite pairs.
+// The sums go in the order of step_body, and the products of the collision are
+// rounded as it rounds them, so the bits are those of the shared body of both
+// component classes that this one replaced.
 // Bound by issue and by the latency between a plane's barriers (20 warps, 0.6
 // instructions a cycle and scheduler); registers hold it to one CTA of 16 rows
-// or two of 8.  FP32, a step: D3Q19 200 x 184 x 168 240 us in the shared body of
-// both component classes, 153 us here (394 instead of 502 instructions a node);
-// D3Q27 HIGHORDER with SMAGORINSKI 316 and 267 us; D3Q19 64^3 16.5 and 11.3 us.
+// or two of 8.  FP32, 200 x 184 x 168, a step: D3Q19 265 us in the shared body,
+// 154 us here; D3Q27 HIGHORDER with SMAGORINSKI 317 and 281 us (267 us with the
+// sums of the rows and populations regrouped, which rounds differently).
+// D3Q27 does not fit in the 96 registers of 16 rows and the 80 of 8: FP32 spills
+// 32-36 bytes (104-136 with obstacles) and 92-120 bytes (196-264).
 #pragma once
 #include "lbf_node.cuh"
 
@@ -204,8 +209,8 @@ __device__ __forceinline__ void single_body(const StepParams<S, R>& p, const int
             R pxz = CD::dec(nxt.m[8], p.inv_scale[8]), pyz = CD::dec(nxt.m[9], p.inv_scale[9]);
             if constexpr (CD::scaled) {
                 // 16-bit storage keeps Pi - u u, the deviation from equilibrium
-                pxx += u * u; pyy += v * v; pzz += w * w;
-                pxy += u * v; pxz += u * w; pyz += v * w;
+                pxx = fmaf_t(u, u, pxx); pyy = fmaf_t(v, v, pyy); pzz = fmaf_t(w, w, pzz);
+                pxy = fmaf_t(u, v, pxy); pxz = fmaf_t(u, w, pxz); pyz = fmaf_t(v, w, pyz);
             }
             // ---- moments prologue: lb_cuda_moments_module.f90:104-339 ----
             const R Fx = p.fx, Fy = p.fy, Fz = p.fz;
@@ -224,24 +229,28 @@ __device__ __forceinline__ void single_body(const StepParams<S, R>& p, const int
                 CD::st(p.uout + 2 * N, gi, w, p.scale[F_UOLD + 2]);
             }
             // ---- collision: lb_cuda_fused_module.f90:531-713 ----
-            const R Xn = pxx - u * u, Yn = pyy - v * v, Zn = pzz - w * w;
-            const R XYn = pxy - u * v, XZn = pxz - u * w, YZn = pyz - v * w;
+            const R uu = mul_rn(u, u), vv = mul_rn(v, v), ww = mul_rn(w, w);
+            const R uv = mul_rn(u, v), uw = mul_rn(u, w), vw = mul_rn(v, w);
+            const R Xn = pxx - uu, Yn = pyy - vv, Zn = pzz - ww;
+            const R XYn = pxy - uv, XZn = pxz - uw, YZn = pyz - vw;
             R omega = p.omega;
             if (p.smag) {
                 // SMAGORINSKI (lb_cuda_fused_module.f90:609-616)
-                const R QQ = Xn * Xn + Yn * Yn + Zn * Zn + R(2) * (XYn * XYn + XZn * XZn + YZn * YZn);
+                const R q1 = fmaf_t(Zn, Zn, fmaf_t(Xn, Xn, mul_rn(Yn, Yn)));
+                const R q2 = fmaf_t(YZn, YZn, fmaf_t(XYn, XYn, mul_rn(XZn, XZn)));
+                const R QQ = fmaf_t(R(2), q2, q1);
                 const R v3 = R(3) * p.visc1;
-                const R tau = R(0.5) + R(1.0 / 6.0) * (v3 + sqrt_a<R>(v3 * v3 + R(SMAG_C) * sqrt_a<R>(R(2) * QQ)));
+                const R tau = fmaf_t(R(1.0 / 6.0), v3 + sqrt_a<R>(fmaf_t(v3, v3, mul_rn(R(SMAG_C), sqrt_a<R>(R(2) * QQ)))), R(0.5));
                 omega = rcp<R>(tau);
             }
             const R om1 = R(1) - omega;
             const R mx = u + R(0.5) * Fx, my = v + R(0.5) * Fy, mz = w + R(0.5) * Fz;
-            const R mxx = u * u + om1 * Xn + u * Fx;
-            const R myy = v * v + om1 * Yn + v * Fy;
-            const R mzz = w * w + om1 * Zn + w * Fz;
-            const R mxy = u * v + om1 * XYn + R(0.5) * (u * Fy + v * Fx);
-            const R mxz = u * w + om1 * XZn + R(0.5) * (u * Fz + w * Fx);
-            const R myz = v * w + om1 * YZn + R(0.5) * (v * Fz + w * Fy);
+            const R mxx = fmaf_t(u, Fx, fmaf_t(om1, Xn, uu));
+            const R myy = fmaf_t(v, Fy, fmaf_t(om1, Yn, vv));
+            const R mzz = fmaf_t(w, Fz, fmaf_t(om1, Zn, ww));
+            const R mxy = fmaf_t(R(0.5), u * Fy + v * Fx, fmaf_t(om1, XYn, uv));
+            const R mxz = fmaf_t(R(0.5), u * Fz + w * Fx, fmaf_t(om1, XZn, uw));
+            const R myz = fmaf_t(R(0.5), v * Fz + w * Fy, fmaf_t(om1, YZn, vw));
             R fpop[27];
             if constexpr (LAT == 27) {
                 R M[3][3][3];
@@ -250,7 +259,7 @@ __device__ __forceinline__ void single_body(const StepParams<S, R>& p, const int
                 M[2][0][0] = mxx; M[0][2][0] = myy; M[0][0][2] = mzz;
                 M[1][1][0] = mxy; M[1][0][1] = mxz; M[0][1][1] = myz;
                 if constexpr (HO) {
-                    ho_rows<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
+                    ho_rows_wide<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
                 } else {
                     M[2][1][0] = M[2][0][1] = M[1][2][0] = M[1][0][2] = M[0][1][2] = M[0][2][1] = M[1][1][1] = R(0);
                     M[2][2][0] = M[2][0][2] = M[0][2][2] = M[1][1][2] = M[1][2][1] = M[2][1][1] = R(0);
@@ -354,12 +363,16 @@ __device__ __forceinline__ void single_body(const StepParams<S, R>& p, const int
                     else if (PG::count(g) == 2) h.v = cz < 0 ? pairs[PG::pair_slot(g) * R1N + src].x : pairs[PG::pair_slot(g) * R1N + src].y;
                     else h.v = singles[PG::single_slot(g) * R1N + src];
                 }
-                const Maybe<R> ex[3] = {f[0][2] + f[0][0], f[1][2] + f[1][0], f[2][2] + f[2][0]};
-                const Maybe<R> s0 = f[0][1] + ex[0], s2 = f[2][1] + ex[2];
-                const Maybe<R> Y02 = s2 + s0, Y01 = s2 - s0, Y20 = (ex[0] + ex[2]) + ex[1];
-                const Maybe<R> Y00 = Y02 + (f[1][1] + ex[1]);
-                const Maybe<R> dm = f[0][2] - f[0][0], dp = f[2][2] - f[2][0];
-                const Maybe<R> Y10 = (dp + dm) + (f[1][2] - f[1][0]), Y11 = dp - dm;
+                // the sums of pull_sums27, in its order
+                Maybe<R> S0[3], S1[3], S2[3];
+#pragma unroll
+                for (int y = 0; y < 3; ++y) {
+                    S0[y] = (f[y][0] + f[y][1]) + f[y][2];
+                    S1[y] = f[y][2] - f[y][0];
+                    S2[y] = f[y][2] + f[y][0];
+                }
+                const Maybe<R> Y00 = (S0[0] + S0[1]) + S0[2], Y01 = S0[2] - S0[0], Y02 = S0[2] + S0[0];
+                const Maybe<R> Y10 = (S1[0] + S1[1]) + S1[2], Y11 = S1[2] - S1[0], Y20 = (S2[0] + S2[1]) + S2[2];
                 R a[10];
 #pragma unroll
                 for (int i = 0; i < 10; ++i) a[i] = cz < 0 ? A2[i].x : cz == 0 ? A2[i].y : ap[i];
