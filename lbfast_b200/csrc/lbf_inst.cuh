@@ -127,9 +127,9 @@ template <int LAT, bool HO, typename S, typename R, int TYV, int OBS> StepLaunch
                         : &launch_stream<LAT, HO, false, S, R, TYV, false, OBS>;
 }
 template <int LAT, bool HO, typename S, typename R, int TYV> StepLauncher step_class(int tc, int obs) {
-    // the correction without obstacles and without REPULSIVE_FLUX is a class of
-    // its own; with REPULSIVE_FLUX the obstacle compilation serves
-    if (obs == 2 && tc == 1) return &launch_stream<LAT, HO, true, S, R, TYV, false, 2>;
+    // (one component has no correction)
+    if (obs == 2 && tc)
+        return tc == 2 ? &launch_stream<LAT, HO, true, S, R, TYV, true, 2> : &launch_stream<LAT, HO, true, S, R, TYV, false, 2>;
     return obs ? step_class<LAT, HO, S, R, TYV, 1>(tc) : step_class<LAT, HO, S, R, TYV, 0>(tc);
 }
 template <typename S, typename R, int TYV> StepLauncher step_table(int lat, int ho, int tc, int obs) {
@@ -147,16 +147,20 @@ template <int LAT, bool HO, typename S, typename R, int TYV, int OBS> void batch
     } else if (tc) {
         o.launch = &launch_stream_batched<LAT, HO, true, S, R, TYV, false, OBS>;
         o.resident = &batched_resident<LAT, HO, true, S, R, TYV, false, OBS>;
-    } else {
+    } else if constexpr (OBS != 3) {
         o.launch = &launch_stream_batched<LAT, HO, false, S, R, TYV, false, OBS>;
         o.resident = &batched_resident<LAT, HO, false, S, R, TYV, false, OBS>;
     }
 }
-// The batched kernels keep obstacles a run-time flag (OBS = 1 for every
+// The batched kernels keep obstacles a run-time flag (odd OBS for every
 // box): the obstacle-free compilation of the batched kernel, unlike the
 // single-box one, ran the droplet-ensemble server slower and erratically
-// (3.2-5.2 against a steady 5.5 solves/s, interleaved runs on one box).
-template <int LAT, bool HO, typename S, typename R, int TYV> void batch_class(int tc, int, BatchOps& o) {
+// (3.2-5.2 against a steady 5.5 solves/s, interleaved runs on one box).  With
+// two components and HIGHORDER, boxes with and without obstacles have the form
+// of the rows that lbf_step gives them.
+template <int LAT, bool HO, typename S, typename R, int TYV> void batch_class(int tc, int obs, BatchOps& o) {
+    if constexpr (HO)
+        if (tc && !obs) return batch_class<LAT, HO, S, R, TYV, 3>(tc, o);
     batch_class<LAT, HO, S, R, TYV, 1>(tc, o);
 }
 template <typename S, typename R, int TYV> BatchOps batch_table(int lat, int ho, int tc, int obs) {

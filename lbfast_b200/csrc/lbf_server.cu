@@ -18,10 +18,11 @@
 // and its device memory is released at the end of the chunk in which it
 // finished, which lets the next queued solves in.
 //
-// Each solve's arithmetic is the single-box kernel's (the same device
-// function, step_body, with the same parameters), so a solve's result does not
-// depend on the other resident solves, nor on the z segmentation the server
-// picks for the batch.
+// Each solve's operations are the single-box kernel's (the same device
+// functions, step_body and single_body, with the same parameters), so a solve's
+// result does not depend on the other resident solves, nor on the z
+// segmentation the server picks for the batch, and agrees with lbf_step's to
+// rounding (another compilation of the same operations).
 #include <cuda_runtime.h>
 #include <time.h>
 

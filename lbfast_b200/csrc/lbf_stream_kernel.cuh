@@ -53,10 +53,13 @@ template <typename S, typename R, int TYV> constexpr size_t stream_smem_bytes() 
 // One piece of a time step: tile (bx, by) of the box, planes z0 <= z < z1.
 // REP: REPULSIVE_FLUX force in the moments prologue; OBS: 1 obstacles (isfluid
 // tests, the moment-space bounce-back) and the phi mass correction, 2 the
-// correction alone, 0 neither.  Separate compilations, so the kernels without
+// correction alone, 0 neither; 3 the code of 1 for a box without obstacles (a
+// batch's), which takes the HIGHORDER rows in the form that such a box steps
+// with alone.  Separate compilations, so the kernels without
 // them carry no code for them: the obstacle code alone, never executed, costs a
 // box without obstacles 5.6 %, and the correction in that compilation a quarter
-// of the step (150 x 128 x 136: 257 us with its sum, 212 us now).
+// of the step (150 x 128 x 136: 257 us with its sum, 214 us in a compilation of
+// its own).
 template <int LAT, bool HO, typename S, typename R, int TYV, bool REP, int OBS>
 __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int bx, const int by, const int z0,
                                           const int z1) {
@@ -98,7 +101,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     const int plane = (int)p.plane;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const bool dr = p.densratio != 0;
-    const bool obs = OBS == 1 && p.obstacles != 0;
+    const bool obs = (OBS & 1) && p.obstacles != 0;
     const R cssq = R(1.0 / 3.0);
 
     // ---- static per-thread node tables (x/y wrap does not change along z) ----
@@ -678,7 +681,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
                     M[2][0][0] = mxx; M[0][2][0] = myy; M[0][0][2] = mzz;
                     M[1][1][0] = mxy; M[1][0][1] = mxz; M[0][1][1] = myz;
                     if constexpr (HO) {
-                        if constexpr (OBS != 0) ho_rows<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
+                        if constexpr (OBS == 1) ho_rows<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
                         else ho_rows_wide<R>(M, u, v, w, om1, Xn, Yn, Zn, XYn, XZn, YZn);
                     } else {
                         M[2][1][0] = M[2][0][1] = M[1][2][0] = M[1][0][2] = M[0][1][2] = M[0][2][1] = M[1][1][1] = R(0);
@@ -801,7 +804,7 @@ template <int LAT, bool TC, typename S, typename R, int TYV> constexpr size_t st
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP, int OBS>
 __device__ __forceinline__ void any_body(const StepParams<S, R>& p, int bx, int by, int z0, int z1) {
     if constexpr (TC) step_body<LAT, HO, S, R, TYV, REP, OBS>(p, bx, by, z0, z1);
-    else single_body<LAT, HO, S, R, TYV, OBS == 1>(p, bx, by, z0, z1);
+    else single_body<LAT, HO, S, R, TYV, (OBS & 1) != 0>(p, bx, by, z0, z1);
 }
 
 // Column-planes of the planes zlo .. zlo + nzr - 1 of a box for a tile of
@@ -861,8 +864,10 @@ __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TY
 
 // Many boxes in one launch: CTA i advances box work[i].x over column-planes
 // [work[i].y, work[i].z) of that box (column-major: plane fastest), with the
-// box's own parameters and fields.  Each node's arithmetic is the same as in
-// stream_kernel, so a box gives the same bits alone and in a batch.
+// box's own parameters and fields.  A box gives the same bits whatever else is
+// in the batch.  Each node's operations are those of stream_kernel, but in
+// another compilation, where the compiler contracts the products of the
+// two-component collision differently: the two agree to rounding.
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
 __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>())
     stream_kernel_batched(const StepParams<S, R>* __restrict__ boxes, const int4* __restrict__ work) {

@@ -25,6 +25,7 @@ def classes():
                         if ho and tc and tile == 8 and st in ("f16", "bf16"):
                             continue
                         out.append((st, lat, ho, tc, smag, tile, False))
+        out.append((st, 27, 1, 2, 0, 8, True))
     return out
 
 

@@ -2,8 +2,8 @@
 
 The claim under test: a solve's result is the same whether it runs alone or
 in a mix with other solves of other sizes, classes, step counts and arrival
-times -- bit for bit, since every solve runs the single-box kernel's
-arithmetic -- and the same as the single-box entry point lbf_step; admission
+times -- bit for bit -- and that of the single-box entry point lbf_step to
+rounding, whose operations every solve runs; admission
 respects the memory budget; cancelling a resident solve leaves the others
 untouched.
 """

@@ -45,3 +45,33 @@ def test_one_component(lattice, highorder, smag, box, tile, zseg, storage, solid
     mo, _, _ = o.get_fields()
     fluid = np.abs(isf) == 1
     assert rel_l2(mg, mo, fluid) < (1e-10 if storage == "f64" else 1e-5)
+
+
+@pytest.mark.parametrize("lattice,highorder", [(15, 0), (19, 0), (27, 1)])
+@pytest.mark.parametrize("box,tile,zseg", [((33, 17, 9), 16, 0), ((31, 15, 5), 8, 2), ((65, 8, 13), 16, -4)])
+@pytest.mark.parametrize("storage,half_ulp", [("f16", 2.0 ** -12), ("bf16", 2.0 ** -9)])
+def test_one_component_16_bit(lattice, highorder, box, tile, zseg, storage, half_ulp):
+    """With walls and a solid block.  Every step rounds the six stored Pi - u u
+    by at most half an ulp; what it changes relaxes in the steps after it: at
+    most `steps` half ulps of the result (P and u are kept in 32 bits)."""
+    lx, ly, lz = box
+    steps = 5
+    p = Params(lx=lx, ly=ly, lz=lz, pbc_y=0, lattice=lattice, highorder=highorder, obstacles=1, visc1=0.05, fx=1e-5,
+               storage=storage, tile_y=tile, zseg=zseg)
+    rng = np.random.default_rng(lx * 1000 + ly * 10 + lz)
+    block = np.zeros(p.shape, dtype=bool)
+    block[1:3, 2:4, 1:4] = True
+    isf = O.mark_isfluid(block, (1, 0, 1), lattice, True)
+    m = np.where((isf == 0)[None], 0.0, _random_moments(rng, p.shape))
+    s = Solver(p)
+    s.set_isfluid(isf)
+    s.set_fields(m)
+    s.step(steps)
+    mg, _, _ = s.get_fields()
+    s.close()
+    o = O.Oracle(p.oracle_dict(), "f64")
+    o.set_isfluid(isf)
+    o.set_fields(m, None)
+    o.step(steps)
+    mo, _, _ = o.get_fields()
+    assert rel_l2(mg, mo, np.abs(isf) == 1) < steps * half_ulp

@@ -61,3 +61,47 @@ def test_wall_passes(box, pbc, bb, types, lattice, highorder):
     isf = O.mark_isfluid(solid, pbc, lattice, True)
     m = np.where((isf == 0)[None], 0.0, _random_moments(rng, p.shape, amp_u=0.003, amp_p=0.002))
     _compare(p, isf, m, None, 4)
+
+
+@pytest.mark.parametrize("box,pbc,corr", [((17, 16, 9), (1, 0, 1), 0), ((33, 10, 15), (1, 0, 1), 1), ((16, 17, 8), (0, 1, 1), 1),
+                                          ((31, 9, 17), (1, 1, 1), 1)])
+def test_film_search_around_solid_nodes(box, pbc, corr):
+    """Solid nodes across the edges of the search's tiles, with and without the mass correction."""
+    lx, ly, lz = box
+    rng = np.random.default_rng(lx * 100 + ly)
+    p = Params(lx=lx, ly=ly, lz=lz, pbc_x=pbc[0], pbc_y=pbc[1], pbc_z=pbc[2], lattice=27, twocomponent=1, densratio=1,
+               visc1=0.05, visc2=0.08, rho_r=1.0, rho_b=0.5, sigma=0.01, width=2.5, tau_diff=0.1, storage="f64",
+               repulsive_flux=1, a_rep=0.05, cos_opp_t=-0.2, q_th=0.02, obstacles=1, phi_correction=corr)
+    solid = np.zeros(p.shape, dtype=bool)
+    solid[6:9, 6:9, 14:18] = True
+    isf = O.mark_isfluid(solid, pbc, 27, True)
+    phi = np.where(isf == 0, 0.0, _blobs(rng, p.shape, 6, 2.0, 4.0, 2.5))
+    m = np.where((isf == 0)[None], 0.0, _random_moments(rng, p.shape, amp_u=0.002, amp_p=0.0005, amp_neq=1e-6))
+    _compare(p, isf, m, phi, 4)
+
+
+@pytest.mark.parametrize("two,bb", [(0, 0), (0, 1), (1, 0)])
+def test_second_set_isfluid(two, bb):
+    """The wall links and wetting tables are those of the last isfluid, with more or fewer wall nodes than before."""
+    extra = dict(twocomponent=1, densratio=1, visc2=0.08, rho_r=1.0, rho_b=0.5, sigma=0.01, width=2.5, tau_diff=0.1) if two else {}
+    p = Params(lx=34, ly=12, lz=10, pbc_y=0, lattice=19, obstacles=1, bounce_back=bb, visc1=0.05, fx=1e-5, storage="f32", **extra)
+    rng = np.random.default_rng(4)
+    m, phi = _random_moments(rng, p.shape), _blobs(rng, p.shape, 3, 2.0, 3.0, 2.5)
+    solid = np.zeros(p.shape, dtype=bool)
+    few = O.mark_isfluid(solid, (1, 0, 1), 19, True)
+    solid[3:7, 4:8, 5:30] = True
+    many = O.mark_isfluid(solid, (1, 0, 1), 19, True)
+
+    def run(geometries):
+        s = Solver(p)
+        for isf in geometries:
+            s.set_isfluid(isf)
+            s.set_fields(np.where((isf == 0)[None], 0.0, m), phi if two else None)
+            s.step(3)
+        out = s.get_fields()
+        s.close()
+        return out
+
+    for a, b in ((few, many), (many, few)):
+        for x, y in zip(run([a, b]), run([b])):
+            assert (x is None and y is None) or np.array_equal(x, y, equal_nan=True)
