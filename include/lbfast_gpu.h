@@ -130,7 +130,9 @@ int lbf_destroy(lbf_handle* h);
 int lbf_set_stream(lbf_handle* h, void* cuda_stream);
 
 /* isfluid as produced by LBFAST.f90:258-325 (values 1, -1, 0; int8, lx*ly*lz,
- * Fortran order).  Required when obstacles = 1; otherwise all nodes are fluid. */
+ * Fortran order).  Required when obstacles = 1; otherwise all nodes are fluid.
+ * May be called again.  After a call that failed the handle has no geometry:
+ * lbf_set_fields and lbf_step return LBF_E_STATE until one succeeds. */
 int lbf_set_isfluid(lbf_handle* h, const int8_t* isfluid);
 
 /* Initial state, replacing the host->device mirror of hfields_flip /
@@ -389,7 +391,8 @@ int lbf_server_fetch(lbf_server* s, long long id, void* mom10, void* phi);
 /* Drops a queued or resident solve; its device memory goes back to the
  * server's pool at once. */
 int lbf_server_cancel(lbf_server* s, long long id);
-/* Device bytes a solve of these parameters holds while resident. */
+/* Device bytes a solve of these parameters holds while resident, without the
+ * tables made from its isfluid (wall links, wetting: a few bytes a wall node). */
 long long lbf_server_solve_bytes(const lbf_params* p);
 
 #ifdef __cplusplus

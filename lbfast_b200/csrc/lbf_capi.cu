@@ -15,6 +15,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -87,16 +88,6 @@ int ensure_staging(lbf_handle* h, size_t bytes) {
     if (!dev_alloc(h, h->staging, bytes))
         return fail(LBF_E_NOMEM, "device staging allocation of %zu bytes failed", bytes);
     h->staging_bytes = bytes;
-    return LBF_OK;
-}
-
-// a device table with the values of v in the place of t
-template <typename T> int replace_table(T*& t, const std::vector<T>& v) {
-    cudaFree(t);
-    t = nullptr;
-    if (v.empty()) return LBF_OK;
-    CUDA_TRY(cudaMalloc(&t, v.size() * sizeof(T)));
-    CUDA_TRY(cudaMemcpy(t, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
     return LBF_OK;
 }
 
@@ -502,58 +493,104 @@ int lbf_set_stream(lbf_handle* h, void* s) {
     return LBF_OK;
 }
 
-int lbf_set_isfluid(lbf_handle* h, const int8_t* isf) {
-    if (!h || !isf) return fail(LBF_E_ARG, "lbf_set_isfluid: null argument");
-    const int nx = h->nx, ny = h->ny, nz = h->nz;
-    for (long long i = 0; i < h->N; ++i)
-        if (isf[i] != 0 && isf[i] != 1 && isf[i] != -1) return fail(LBF_E_ARG, "isfluid[%lld] = %d not in {1,-1,0}", i, isf[i]);
-    if (!h->obs) {
-        for (long long i = 0; i < h->N; ++i)
-            if (isf[i] != 1) return fail(LBF_E_ARG, "isfluid has non-fluid nodes but obstacles = 0");
-        return LBF_OK;
-    }
-    CUDA_TRY(cudaMemcpyAsync(h->isf, isf, h->N, cudaMemcpyHostToDevice, h->stream));
-    h->isf_set = true;
-    const int pb[3] = {h->p.pbc_x, h->p.pbc_y, h->p.pbc_z};
-    const int dims[3] = {nx, ny, nz};
-    const int lat = h->p.lattice;
-    auto isf_at = [&](int x, int y, int z) -> int {
+}  // extern "C"
+
+namespace {
+
+// isfluid of a node, folded into the box on periodic axes; never-written halo keeps 1
+struct IsfAt {
+    const int8_t* isf;
+    int n[3], pb[3];
+    IsfAt(const lbf_handle* h, const int8_t* f) : isf(f), n{h->nx, h->ny, h->nz}, pb{h->p.pbc_x, h->p.pbc_y, h->p.pbc_z} {}
+    int operator()(int x, int y, int z) const {
         int c[3] = {x, y, z};
         for (int d = 0; d < 3; ++d) {
-            if (c[d] < 0 || c[d] >= dims[d]) {
-                if (!pb[d]) return 1;  // never-written halo keeps isfluid = 1
-                c[d] = (c[d] % dims[d] + dims[d]) % dims[d];
+            if (c[d] < 0 || c[d] >= n[d]) {
+                if (!pb[d]) return 1;
+                c[d] = (c[d] % n[d] + n[d]) % n[d];
             }
         }
-        return isf[((long long)c[2] * ny + c[1]) * nx + c[0]];
-    };
-    // wall links of every isfluid = -1 node (bit l: the upstream node x - c_l is
-    // solid), row by row in the step kernel's 32-wide x segments; and the nodes
-    // whose links the passes after the step rewrite: BOUNCE_BACK every -1 node
-    // (of a slab's own planes), the open faces theirs
-    {
-        const int segs = (nx + lbf::STEP_TILE_X - 1) / lbf::STEP_TILE_X;
-        const int k_lo = h->slab ? lbf::SLAB_HALO : 0, k_hi = h->slab ? lbf::SLAB_HALO + h->nzs : nz;
-        const bool passes = h->p.bounce_back || h->obc_open;
-        std::vector<int> rows((size_t)nz * ny * segs);
-        std::vector<unsigned> links, wall_links;
-        std::vector<long long> wall_nodes;
-        long long up[27];
-        for (int l = 0; l < 27; ++l) up[l] = -(((long long)EZh[l] * ny + EYh[l]) * nx + EXh[l]);
-        for (int k = 0; k < nz; ++k)
-            for (int j = 0; j < ny; ++j) {
-                const int8_t* row = isf + ((long long)k * ny + j) * nx;
-                const bool edge = k == 0 || k == nz - 1 || j == 0 || j == ny - 1;
-                for (int i = 0; i < nx; ++i) {
-                    if (i % lbf::STEP_TILE_X == 0)
-                        rows[((size_t)k * ny + j) * segs + i / lbf::STEP_TILE_X] = (int)links.size();
-                    if (row[i] != -1) continue;
+        return isf[((long long)c[2] * n[1] + c[1]) * n[0] + c[0]];
+    }
+};
+
+// Device tables made from isfluid.  They are built apart from the handle's and
+// change places with them once every allocation and copy has succeeded: the
+// step kernels read them without a test.
+struct IsfTables {
+    int* link_rows = nullptr;
+    unsigned *links = nullptr, *wall_links = nullptr;
+    long long *wall_nodes = nullptr, *wet_s = nullptr;
+    int *wet_donor = nullptr, *wet_flag = nullptr, *wet_shift = nullptr;
+    double* wet_wn = nullptr;
+    void* wetW[2] = {nullptr, nullptr};
+    long long nwall = 0;
+    int nwet = 0;
+    ~IsfTables() {
+        for (void* q : {(void*)link_rows, (void*)links, (void*)wall_links, (void*)wall_nodes, (void*)wet_s, (void*)wet_donor,
+                        (void*)wet_flag, (void*)wet_shift, (void*)wet_wn, wetW[0], wetW[1]})
+            if (q) cudaFree(q);
+    }
+    void swap(lbf_handle* h) {
+        std::swap(link_rows, h->link_rows);
+        std::swap(links, h->links);
+        std::swap(wall_links, h->wall_links);
+        std::swap(wall_nodes, h->wall_nodes);
+        std::swap(wet_s, h->wet_s);
+        std::swap(wet_donor, h->wet_donor);
+        std::swap(wet_flag, h->wet_flag);
+        std::swap(wet_shift, h->wet_shift);
+        std::swap(wet_wn, h->wet_wn);
+        std::swap(wetW[0], h->wetW[0]);
+        std::swap(wetW[1], h->wetW[1]);
+        std::swap(nwall, h->nwall);
+        std::swap(nwet, h->nwet);
+    }
+};
+// (in order with the handle's kernels; v has to live until its stream is synchronised)
+template <typename T> int upload_table(const lbf_handle* h, T*& t, const std::vector<T>& v) {
+    if (v.empty()) return LBF_OK;
+    CUDA_TRY(cudaMalloc(&t, v.size() * sizeof(T)));
+    CUDA_TRY(cudaMemcpyAsync(t, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
+    return LBF_OK;
+}
+
+// wall links of every isfluid = -1 node (bit l: the upstream node x - c_l is
+// solid), row by row in the step kernel's 32-wide x segments; and the nodes
+// whose links the passes after the step rewrite: BOUNCE_BACK every -1 node
+// (of a slab's own planes), the open faces theirs
+int link_tables(const lbf_handle* h, const int8_t* isf, IsfTables& t) {
+    const int nx = h->nx, ny = h->ny, nz = h->nz, lat = h->p.lattice;
+    const int dims[3] = {nx, ny, nz};
+    const IsfAt isf_at(h, isf);
+    const int segs = (nx + lbf::STEP_TILE_X - 1) / lbf::STEP_TILE_X;
+    const int k_lo = h->slab ? lbf::SLAB_HALO : 0, k_hi = h->slab ? lbf::SLAB_HALO + h->nzs : nz;
+    const bool passes = h->p.bounce_back || h->obc_open;
+    std::vector<int> rows((size_t)nz * ny * segs);
+    std::vector<unsigned> links, wall_links;
+    std::vector<long long> wall_nodes;
+    int ls[27], nl = 0;  // the links of the lattice
+    long long up[27];
+    for (int l = 1; l < 27; ++l) {
+        if (!link_in(lat, l)) continue;
+        ls[nl++] = l;
+        up[l] = -(((long long)EZh[l] * ny + EYh[l]) * nx + EXh[l]);
+    }
+    for (int k = 0; k < nz; ++k)
+        for (int j = 0; j < ny; ++j) {
+            const int8_t* row = isf + ((long long)k * ny + j) * nx;
+            const bool edge = k == 0 || k == nz - 1 || j == 0 || j == ny - 1;
+            for (int x0 = 0; x0 < nx; x0 += lbf::STEP_TILE_X) {
+                rows[((size_t)k * ny + j) * segs + x0 / lbf::STEP_TILE_X] = (int)links.size();
+                const int8_t* const end = row + std::min(nx, x0 + lbf::STEP_TILE_X);
+                // the -1 nodes of the segment
+                for (const int8_t* q = row + x0; (q = static_cast<const int8_t*>(std::memchr(q, 0xff, end - q))); ++q) {
+                    const int i = (int)(q - row);
+                    const bool fold = edge || i == 0 || i == nx - 1;
                     unsigned m = 0;
-                    for (int l = 1; l < 27; ++l) {
-                        if (!link_in(lat, l)) continue;
-                        const int f = edge || i == 0 || i == nx - 1 ? isf_at(i - EXh[l], j - EYh[l], k - EZh[l])
-                                                                    : row[i + up[l]];
-                        if (f == 0) m |= 1u << l;
+                    for (int n = 0; n < nl; ++n) {
+                        const int l = ls[n], f = fold ? isf_at(i - EXh[l], j - EYh[l], k - EZh[l]) : q[up[l]];
+                        m |= (unsigned)(f == 0) << l;
                     }
                     links.push_back(m);
                     if (!passes || !m || k < k_lo || k >= k_hi) continue;
@@ -561,20 +598,26 @@ int lbf_set_isfluid(lbf_handle* h, const int8_t* isf) {
                     bool take = h->p.bounce_back != 0;
                     for (int f = 0; f < 6 && !take; ++f) take = lbf::open_face_node(h->obc_open, at, dims, f >> 1, f & 1);
                     if (!take) continue;
-                    wall_nodes.push_back(row - isf + i);
+                    wall_nodes.push_back(q - isf);
                     wall_links.push_back(m);
                 }
             }
-        int rc = replace_table(h->link_rows, rows);
-        if (!rc) rc = replace_table(h->links, links);
-        if (!rc) rc = replace_table(h->wall_nodes, wall_nodes);
-        if (!rc) rc = replace_table(h->wall_links, wall_links);
-        if (rc) return rc;
-        h->nwall = (long long)wall_nodes.size();
-    }
-    if (!h->tc) return LBF_OK;
-    // wetting tables: PHI_int_boundary_kernel steps 1-2 (lb_cuda_boundary_module.f90:281-398),
-    // in double; they depend on isfluid only.
+        }
+    t.nwall = (long long)wall_nodes.size();
+    int rc = upload_table(h, t.link_rows, rows);
+    if (!rc) rc = upload_table(h, t.links, links);
+    if (!rc) rc = upload_table(h, t.wall_nodes, wall_nodes);
+    if (!rc) rc = upload_table(h, t.wall_links, wall_links);
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return rc;
+}
+
+// wetting tables: PHI_int_boundary_kernel steps 1-2 (lb_cuda_boundary_module.f90:281-398),
+// in double; they depend on isfluid only.
+int wet_tables(const lbf_handle* h, const int8_t* isf, IsfTables& t) {
+    const int nx = h->nx, ny = h->ny, nz = h->nz, lat = h->p.lattice;
+    const int dims[3] = {nx, ny, nz}, pb[3] = {h->p.pbc_x, h->p.pbc_y, h->p.pbc_z};
+    const IsfAt isf_at(h, isf);
     std::vector<long long> vs;
     std::vector<int> vd, vf, vsh;
     std::vector<double> vwn;
@@ -671,26 +714,51 @@ int lbf_set_isfluid(lbf_handle* h, const int8_t* isf) {
                     }
         }
     }
-    cudaFree(h->wet_s); cudaFree(h->wet_donor); cudaFree(h->wet_flag); cudaFree(h->wet_wn); cudaFree(h->wet_shift);
-    cudaFree(h->wetW[0]); cudaFree(h->wetW[1]);
-    h->wet_s = nullptr; h->wet_donor = nullptr; h->wet_flag = nullptr; h->wet_wn = nullptr; h->wet_shift = nullptr;
-    h->wetW[0] = h->wetW[1] = nullptr;
-    h->nwet = (int)vs.size();
-    h->wet_pending = -1;
-    if (h->nwet == 0) return LBF_OK;
-    CUDA_TRY(cudaMalloc(&h->wet_s, vs.size() * sizeof(long long)));
-    CUDA_TRY(cudaMalloc(&h->wet_donor, vd.size() * sizeof(int)));
-    CUDA_TRY(cudaMalloc(&h->wet_flag, vf.size() * sizeof(int)));
-    CUDA_TRY(cudaMalloc(&h->wet_wn, vwn.size() * sizeof(double)));
-    CUDA_TRY(cudaMalloc(&h->wet_shift, vsh.size() * sizeof(int)));
-    CUDA_TRY(cudaMalloc(&h->wetW[0], h->nwet * h->psz));
-    CUDA_TRY(cudaMalloc(&h->wetW[1], h->nwet * h->psz));
-    CUDA_TRY(cudaMemcpy(h->wet_s, vs.data(), vs.size() * sizeof(long long), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(h->wet_donor, vd.data(), vd.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(h->wet_flag, vf.data(), vf.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(h->wet_wn, vwn.data(), vwn.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(h->wet_shift, vsh.data(), vsh.size() * sizeof(int), cudaMemcpyHostToDevice));
+    t.nwet = (int)vs.size();
+    if (t.nwet == 0) return LBF_OK;
+    int rc = upload_table(h, t.wet_s, vs);
+    if (!rc) rc = upload_table(h, t.wet_donor, vd);
+    if (!rc) rc = upload_table(h, t.wet_flag, vf);
+    if (!rc) rc = upload_table(h, t.wet_wn, vwn);
+    if (!rc) rc = upload_table(h, t.wet_shift, vsh);
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (rc) return rc;
+    for (void*& w : t.wetW) CUDA_TRY(cudaMalloc(&w, t.nwet * h->psz));
     return LBF_OK;
+}
+
+int set_isfluid(lbf_handle* h, const int8_t* isf) {
+    // without a complete set of tables the handle has no geometry: it takes no step
+    h->isf_set = false;
+    IsfTables t;
+    int rc = link_tables(h, isf, t);
+    if (!rc && h->tc) rc = wet_tables(h, isf, t);
+    if (rc) return rc;
+    t.swap(h);  // t holds, and frees, the tables of an earlier call
+    h->wet_pending = -1;
+    CUDA_TRY(cudaMemcpyAsync(h->isf, isf, h->N, cudaMemcpyHostToDevice, h->stream));
+    h->isf_set = true;
+    return LBF_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int lbf_set_isfluid(lbf_handle* h, const int8_t* isf) {
+    if (!h || !isf) return fail(LBF_E_ARG, "lbf_set_isfluid: null argument");
+    for (long long i = 0; i < h->N; ++i)
+        if (isf[i] != 0 && isf[i] != 1 && isf[i] != -1) return fail(LBF_E_ARG, "isfluid[%lld] = %d not in {1,-1,0}", i, isf[i]);
+    if (!h->obs) {
+        for (long long i = 0; i < h->N; ++i)
+            if (isf[i] != 1) return fail(LBF_E_ARG, "isfluid has non-fluid nodes but obstacles = 0");
+        return LBF_OK;
+    }
+    try {
+        return set_isfluid(h, isf);
+    } catch (const std::bad_alloc&) {
+        return fail(LBF_E_NOMEM, "lbf_set_isfluid: host allocation failed");
+    }
 }
 
 int lbf_set_fields(lbf_handle* h, const void* mom10, const void* phi, int dtype) {
@@ -777,6 +845,7 @@ int lbf_step(lbf_handle* h, int nsteps) {
     if (!h) return fail(LBF_E_ARG, "lbf_step: null handle");
     if (nsteps < 0) return fail(LBF_E_ARG, "nsteps < 0");
     if (!h->fields_set) return fail(LBF_E_STATE, "lbf_step before lbf_set_fields");
+    if (h->obs && !h->isf_set) return fail(LBF_E_STATE, "lbf_step: the last lbf_set_isfluid failed");
     if (!h->primed) {
         int rc = prime(h);
         if (rc) return rc;
@@ -996,6 +1065,8 @@ int check_slabs(lbf_handle* const* slabs, int n, const char* who) {
             slabs[i]->nx != slabs[0]->nx || slabs[i]->ny != slabs[0]->ny)
             return fail(LBF_E_ARG, "%s: slab %d does not match slab 0", who, i);
         if (!slabs[i]->fields_set) return fail(LBF_E_STATE, "%s: slab %d has no fields", who, i);
+        if (slabs[i]->obs && !slabs[i]->isf_set)
+            return fail(LBF_E_STATE, "%s: the last lbf_set_isfluid of slab %d failed", who, i);
     }
     return LBF_OK;
 }

@@ -1,0 +1,79 @@
+"""Host paths around the device, run in a child process against a CUDA runtime
+that keeps device memory on the host and launches nothing (fake_cudart.c):
+allocations that fail, the memory that an admission holds, the keys of the
+schedule cache.  No GPU."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = """
+import ctypes, sys
+sys.path[:0] = [{root!r}, {here!r}]
+import numpy as np
+import lbfast_b200 as L
+from lbfast_b200.capi import LBF_OK
+fake = ctypes.CDLL({so!r})
+fake.fake_launches.restype = fake.fake_peak.restype = ctypes.c_longlong
+E_STATE = {state}
+def code(f, *a, **k):
+    try:
+        f(*a, **k)
+    except L.LbfError as e:
+        return e.code
+    return LBF_OK
+def isfluid(p):
+    f = np.ones(p.shape, np.int8)
+    f[:, 0] = f[:, -1] = 0
+    f[:, 1] = f[:, -2] = -1
+    return f
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-Wall", "-Werror", "-Wno-builtin-declaration-mismatch", "-o", so,
+                    os.path.join(HERE, "fake_cudart.c")], check=True)
+
+    def run(body):
+        pre = PRELUDE.format(root=os.path.dirname(HERE), here=HERE, so=so, state=-4)
+        r = subprocess.run([sys.executable, "-c", pre + body], env=dict(os.environ, LD_PRELOAD=so), capture_output=True,
+                           text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+@pytest.mark.parametrize("extra", ["", ", bounce_back=1", ", twocomponent=1, visc2=0.1, width=4.0"])
+def test_failed_set_isfluid_leaves_no_half_made_geometry(fake, extra):
+    """Whichever of its allocations fails, the handle takes no fields before and
+    no step after, and launches nothing; a call that succeeds sets it right."""
+    fake("""
+p = L.Params(lx=40, ly=12, lz=9, lattice=19, obstacles=1, pbc_y=0, visc1=0.1, storage="f32", tile_y=16%s)
+f = isfluid(p)
+m, phi = np.zeros((10,) + p.shape, np.float32), np.zeros(p.shape, np.float32) if p.twocomponent else None
+failed = 0
+for n in range(40):
+    s = L.Solver(p)
+    fake.fake_fail_alloc(n)
+    rc = code(s.set_isfluid, f)
+    fake.fake_fail_alloc(-1)
+    if rc == LBF_OK:
+        s.close()
+        break
+    failed += 1
+    assert code(s.set_fields, m, phi) == E_STATE
+    assert code(s.set_isfluid, f) == LBF_OK and code(s.set_fields, m, phi) == LBF_OK and code(s.step, 2) == LBF_OK
+    # once more, with tables in place
+    fake.fake_fail_alloc(n)
+    assert code(s.set_isfluid, f) != LBF_OK
+    fake.fake_fail_alloc(-1)
+    before = fake.fake_launches()
+    assert code(s.step, 2) == E_STATE and fake.fake_launches() == before
+    assert code(s.set_isfluid, f) == LBF_OK and code(s.step, 2) == LBF_OK and fake.fake_launches() > before
+    s.close()
+assert failed >= 2, failed
+""" % extra)
