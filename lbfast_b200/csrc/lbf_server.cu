@@ -144,7 +144,8 @@ struct lbf_server {
     // steps (12 solves of 32^3-64^3, 64 steps each, submitted and fetched: 84 ms,
     // 55 ms now).  Unused blocks above the memory budget are given back at each
     // admission, all but POOL_KEEP when the server is idle, the rest when it is
-    // destroyed.
+    // destroyed.  On top of the residents' bytes comes one staging buffer, that of
+    // the solve that is being admitted.
     cudaMemPool_t pool = nullptr;
     long long next_id = 1;
     std::map<long long, std::unique_ptr<Solve>> solves;
@@ -218,7 +219,6 @@ int admit(lbf_server* s) {
         // the solve's state is complete before it joins the steps on `stream`
         if (rc == LBF_OK && cudaStreamSynchronize(s->upload) != cudaSuccess)
             rc = sfail(LBF_E_CUDA, "solve set-up failed");
-        if (rc == LBF_OK) rc = lbf_set_stream(h, s->stream);
         if (rc != LBF_OK) {
             char msg[512];
             lbf_last_error(msg, sizeof msg);
@@ -228,7 +228,10 @@ int admit(lbf_server* s) {
             if (h) lbf_destroy(h);
             continue;
         }
+        // on the upload stream, where the next admission can take the block over
+        // at once: a free on `stream` would wait there for the running chunk
         lbf::handle_release_staging(h);
+        lbf_set_stream(h, s->stream);
         v->h = h;
         v->state = LBF_SOLVE_ACTIVE;
         v->t_admit = now_mono();

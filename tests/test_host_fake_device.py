@@ -77,3 +77,24 @@ for n in range(40):
     s.close()
 assert failed >= 2, failed
 """ % extra)
+
+
+def test_admission_during_a_chunk_holds_one_staging_buffer(fake):
+    """Solves that are admitted while a chunk runs: the device holds the budget
+    and one staging buffer, however many are admitted at once."""
+    fake("""
+p = L.Params(lx=32, ly=32, lz=32, lattice=27, highorder=1, twocomponent=1, densratio=1, visc1=0.1, visc2=0.1,
+             rho_r=2.0, sigma=0.01, width=4.0, tau_diff=0.1, storage="f16")
+m, phi = np.zeros((10,) + p.shape, np.float32), np.zeros(p.shape, np.float32)
+b, staging = L.Server.solve_bytes(p), m.nbytes
+s = L.Server(mem_budget=5 * b + b // 2, chunk=4, use_graph=False)
+fake.fake_reset_peak()
+base = fake.fake_peak()
+long = s.submit(p, m, phi, 40)
+ids = [s.submit(p, m, phi, 4) for _ in range(12)]
+s.drain()
+assert all(s.poll(i)["state"] == "done" for i in [long] + ids)
+held = fake.fake_peak() - base
+assert held <= 5 * b + staging + 65536, (held / b, staging / b)
+s.close()
+""")
