@@ -166,16 +166,19 @@ std::vector<int> split_planes(int nx, int ny, int nzr, int tile_y, int storage) 
 // changes host-side state, is not part of a trial).  The winner is remembered
 // per box shape and class.
 struct TuneKey {
-    int v[12];
-    bool operator<(const TuneKey& o) const { return std::lexicographical_compare(v, v + 12, o.v, o.v + 12); }
+    int v[15];
+    bool operator<(const TuneKey& o) const { return std::lexicographical_compare(v, v + 15, o.v, o.v + 15); }
 };
 std::mutex g_tune_mu;
 std::map<TuneKey, std::pair<int, int>> g_tune_cache;
 
+// what the step's kernel, its work a node and the schedules that are tried depend on
 TuneKey tune_key(const lbf_handle* h) {
     const lbf_params& p = h->p;
-    return TuneKey{{p.storage, p.lattice, p.highorder, p.twocomponent, p.densratio, p.obstacles, p.lx, p.ly, p.lz,
-                    p.pbc_x * 4 + p.pbc_y * 2 + p.pbc_z, p.zseg, p.phi_correction != 0}};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return TuneKey{{p.storage, p.lattice, p.highorder, lbf::kernel_tc(p), lbf::kernel_obs(p), p.densratio, p.smagorinsky,
+                    p.lx, p.ly, p.lz, p.pbc_x * 4 + p.pbc_y * 2 + p.pbc_z, h->slab ? h->nzs : 0, p.zseg, h->tile_y, dev}};
 }
 
 int autotune(lbf_handle* h) {
@@ -242,8 +245,9 @@ int autotune(lbf_handle* h) {
         h->zseg = zs0;
         cudaError_t e = L(a, h->stream);  // warm-up (first use sets the kernel's shared-memory limit)
         float ms = 1e30f;
-        // steps shorter than the launches' jitter are timed three times
-        for (int r = 0; r < 3 && e == cudaSuccess && (r == 0 || ms < 0.3f); ++r) {
+        // steps shorter than the launches' jitter are timed three times, unless
+        // they are far behind
+        for (int r = 0; r < 3 && e == cudaSuccess && (r == 0 || (ms < 0.3f && ms < 1.25f * best)); ++r) {
             float t = 0;
             e = cudaEventRecord(e0, h->stream);
             for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = L(a, h->stream);

@@ -98,3 +98,27 @@ held = fake.fake_peak() - base
 assert held <= 5 * b + staging + 65536, (held / b, staging / b)
 s.close()
 """)
+
+
+def test_schedules_are_tuned_per_kernel_class(fake):
+    """A class of its own times its own schedules: none takes over one that was
+    measured on another kernel of the same box."""
+    fake("""
+base = dict(lx=64, ly=48, lz=40, lattice=27, highorder=1, twocomponent=1, visc1=0.1, visc2=0.1, sigma=0.01, width=4.0,
+            tau_diff=0.1, storage="f32")
+def first_step(**kw):
+    p = L.Params(**dict(base, **kw))
+    s = L.Solver(p)
+    s.set_fields(np.zeros((10,) + p.shape, np.float32), np.zeros(p.shape, np.float32))
+    n = fake.fake_launches()
+    s.step(1)
+    n = fake.fake_launches() - n
+    s.close()
+    return n
+assert first_step() > 10
+assert first_step() < 5  # the same class again
+film = dict(repulsive_flux=1, a_rep=0.05, cos_opp_t=-0.5, q_th=0.05)
+for other in (film, dict(phi_correction=1), dict(smagorinsky=1), dict(film, phi_correction=1)):
+    assert first_step(**other) > 10, other
+    assert first_step(**other) < 8, other
+""")
