@@ -155,7 +155,7 @@ __device__ __forceinline__ void single_body(const StepParams<S, R>& p, const int
         const int gi = wz * plane + off;
         if constexpr (LY::split) {
 #pragma unroll
-            for (int f = 0; f < 4; ++f) nxt.v32[f] = __ldg(p.pres_in + f * N + gi);
+            for (int f = 0; f < 4; ++f) nxt.v32[f] = p.pres_in[f * N + gi];
 #pragma unroll
             for (int f = 4; f < 10; ++f) nxt.m[f] = CD::raw(p.min + LY::off(f, N), gi);
         } else {

@@ -388,7 +388,7 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     auto fetch = [&](int gi, NodeRaw& r) {
         if constexpr (LY::split) {
 #pragma unroll
-            for (int f = 0; f < 4; ++f) r.v32[f] = __ldg(p.pres_in + f * N + gi);
+            for (int f = 0; f < 4; ++f) r.v32[f] = p.pres_in[f * N + gi];
 #pragma unroll
             for (int f = 4; f < 10; ++f) r.m[f] = CD::raw(p.min + LY::off(f, N), gi);
         } else {

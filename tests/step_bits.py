@@ -20,9 +20,11 @@ def classes():
                     for tile in (8, 16):
                         if st == "f64" and tile == 16:
                             continue
-                        # the compiler contracts the two-component HIGHORDER collision of 16-bit
-                        # storage in 8-row tiles in a way of its own from build to build
-                        if ho and tc and tile == 8 and st in ("f16", "bf16"):
+                        # with two components and HIGHORDER in 8-row tiles, which a run takes only
+                        # by name, the compiler contracts the collision in another way from build
+                        # to build: held to the 16-row tiles within 1e-6 (FP32) and 1e-3 (16-bit)
+                        # of the result by test_gpu_parity.py's test of the tile heights
+                        if ho and tc and tile == 8 and st != "f64":
                             continue
                         out.append((st, lat, ho, tc, smag, tile, False))
         out.append((st, 27, 1, 2, 0, 8, True))

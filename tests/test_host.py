@@ -285,3 +285,12 @@ def test_first_extrema_of_a_damped_oscillation():
     assert abs(ex[0][0] - T / 2) < 40 and abs(ex[1][0] - T) < 40 and abs(ex[2][0] - 1.5 * T) < 40, ex
     assert abs((ex[2][0] - ex[0][0]) - T) < 10, ex
     assert ex[2][1] > ex[0][1]
+
+
+def test_non_coherent_loads_are_of_tables_only():
+    """A chained kernel starts while its predecessor writes the fields, so only
+    the wall-link tables, which no kernel writes, may be read with __ldg."""
+    csrc, loads = os.path.join(ROOT, "lbfast_b200", "csrc"), []
+    for f in os.listdir(csrc):
+        loads += re.findall(r"__ldg\((\S+)", re.sub(r"//.*", "", open(os.path.join(csrc, f)).read()))
+    assert loads and all(a.startswith(("p.link_rows", "p.links")) for a in loads), loads
