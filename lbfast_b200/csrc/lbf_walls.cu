@@ -34,6 +34,12 @@ int grid_for(long long n, int bs) {
 }
 
 constexpr int WALL_THREADS = 64;  // a short list still spreads over the SMs
+// CTAs per SM: 168 registers a thread, which hold a node's state (16-bit storage
+// with HIGHORDER spills 12-16 bytes, the others nothing).
+// Left to itself the compiler took 72-128 and spilled 132-260 bytes: two
+// components with BOUNCE_BACK 33 x 150 x 130 D3Q15 1.13 ms a step in passes of
+// their own, 1.42 ms in this kernel with the spills, 1.18 ms now.
+constexpr int WALL_MIN_CTAS = 6;
 
 // factor of axis multiplicity m of the D3Q27 Hermite row r in Minv_mrt(r, l)
 // = w_l prod_axes F(m, c): 1, c / cs^2, (c^2 - cs^2) / (2 cs^4)
@@ -339,12 +345,14 @@ __device__ double collision_omega(const BoundaryArgs& a, const NodeState& ns, co
 // differ by the odd and higher terms only, which are added here.
 //
 // Bound by the latency of a node's FP64 chain: the list is a few per cent of
-// the box.  The solid tests are a bit mask per node, made with the list; they
-// were 26 loads of isfluid with a wrapped index each.  160 x 96 x 80 D3Q19
-// with two open axes and 24 spheres (BOUNCE_BACK and four faces): the step
-// and its wall passes 189 us as five launches, 135 us as one.
+// the box.  With two components the chain holds the stencils of theta, 81 values
+// in local memory, and is ten times as long.  The solid tests are a bit mask per
+// node, made with the list; they were 26 loads of isfluid with a wrapped index
+// each.  160 x 96 x 80 D3Q19 with two open axes and 24 spheres (BOUNCE_BACK and
+// four faces): the step and its wall passes 189 us as five launches, 135 us as
+// one, 62 us with the one-component step body.
 template <typename S, int LAT, bool HO>
-__global__ void __launch_bounds__(WALL_THREADS) wall_kernel(const BoundaryArgs a) {
+__global__ void __launch_bounds__(WALL_THREADS, WALL_MIN_CTAS) wall_kernel(const BoundaryArgs a) {
     const long long plane = (long long)a.nx * a.ny, N = plane * a.nz;
     const double cssq = 1.0 / 3.0;
     chain_begin();
