@@ -140,28 +140,22 @@ template <typename S, typename R, int TYV> StepLauncher step_table(int lat, int 
     return nullptr;
 }
 
-template <int LAT, bool HO, typename S, typename R, int TYV, int OBS> void batch_class(int tc, BatchOps& o) {
-    if (tc == 2) {
-        o.launch = &launch_stream_batched<LAT, HO, true, S, R, TYV, true, OBS>;
-        o.resident = &batched_resident<LAT, HO, true, S, R, TYV, true, OBS>;
-    } else if (tc) {
-        o.launch = &launch_stream_batched<LAT, HO, true, S, R, TYV, false, OBS>;
-        o.resident = &batched_resident<LAT, HO, true, S, R, TYV, false, OBS>;
-    } else if constexpr (OBS != 3) {
-        o.launch = &launch_stream_batched<LAT, HO, false, S, R, TYV, false, OBS>;
-        o.resident = &batched_resident<LAT, HO, false, S, R, TYV, false, OBS>;
-    }
+template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP, int OBS> void batch_kernel(BatchOps& o) {
+    o.launch = &launch_stream_batched<LAT, HO, TC, S, R, TYV, REP, OBS>;
+    o.resident = &batched_resident<LAT, HO, TC, S, R, TYV, REP, OBS>;
 }
-// The batched kernels keep obstacles a run-time flag (odd OBS for every
-// box): the obstacle-free compilation of the batched kernel, unlike the
-// single-box one, ran the droplet-ensemble server slower and erratically
+// The batched kernels of two components keep obstacles a run-time flag (odd OBS
+// for every box): the obstacle-free compilation of the batched kernel, unlike
+// the single-box one, ran the droplet-ensemble server slower and erratically
 // (3.2-5.2 against a steady 5.5 solves/s, interleaved runs on one box).  With
-// two components and HIGHORDER, boxes with and without obstacles have the form
-// of the rows that lbf_step gives them.
+// HIGHORDER, boxes with and without obstacles have the form of the rows that
+// lbf_step gives them.  One component has a compilation without the obstacle
+// code, which costs D3Q27 100 bytes of spills (see solve_tile for the figures).
 template <int LAT, bool HO, typename S, typename R, int TYV> void batch_class(int tc, int obs, BatchOps& o) {
-    if constexpr (HO)
-        if (tc && !obs) return batch_class<LAT, HO, S, R, TYV, 3>(tc, o);
-    batch_class<LAT, HO, S, R, TYV, 1>(tc, o);
+    constexpr int PLAIN = HO ? 3 : 1;
+    if (!tc) return obs ? batch_kernel<LAT, HO, false, S, R, TYV, false, 1>(o) : batch_kernel<LAT, HO, false, S, R, TYV, false, 0>(o);
+    if (tc == 2) return obs ? batch_kernel<LAT, HO, true, S, R, TYV, true, 1>(o) : batch_kernel<LAT, HO, true, S, R, TYV, true, PLAIN>(o);
+    return obs ? batch_kernel<LAT, HO, true, S, R, TYV, false, 1>(o) : batch_kernel<LAT, HO, true, S, R, TYV, false, PLAIN>(o);
 }
 template <typename S, typename R, int TYV> BatchOps batch_table(int lat, int ho, int tc, int obs) {
     BatchOps o;

@@ -125,10 +125,18 @@ struct Batch {
     std::vector<int4> h_work;
 };
 
-// tile height of a solve's class: the one requested, else 8 rows.  A batch of
-// small boxes has few 16-row columns to spread over the SMs (measured on the
-// droplet ensemble: 4.9 solves/s with 8 rows, 4.1 with 16).
-int solve_tile(const lbf_params& p) { return p.tile_y ? p.tile_y : 8; }
+// tile height of a solve's class: the one requested, else with two components 8
+// rows -- a batch of small boxes has few 16-row columns to spread over the SMs
+// (droplet ensemble: 4.9 solves/s with 8 rows, 4.1 with 16) -- and with one
+// component 16, whose kernel has more registers and shorter pieces: twelve boxes
+// of 32^3 to 64^3 of D3Q27 HIGHORDER, FP32, 93 us a step in the body that both
+// component classes shared, 140 us in the one-component body with 8 rows and
+// the obstacle code, 105 us without that, 80 us with 16 rows (D3Q19: 73, 68, 51
+// and 50 us).
+int solve_tile(const lbf_params& p) {
+    if (p.tile_y) return p.tile_y;
+    return !p.twocomponent && lbf::tile_available(p.storage, 16) ? 16 : 8;
+}
 
 }  // namespace
 

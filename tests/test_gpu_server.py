@@ -10,7 +10,7 @@ untouched.
 import numpy as np
 import pytest
 
-from cases import make_case, rel_l2, run_oracle
+from cases import _random_moments, make_case, rel_l2, run_oracle
 import lbfast_b200 as L
 
 pytestmark = pytest.mark.gpu
@@ -86,6 +86,32 @@ def test_server_equals_single_box_entry_point(alone, i):
     assert rel_l2(ms, mg, fl) < bar
     if p.twocomponent:
         assert rel_l2(ps, pg, fl) < bar
+
+
+@pytest.mark.parametrize("storage", ["f32", "bf16", "f64"])
+@pytest.mark.parametrize("lattice,highorder", [(15, 0), (19, 0), (27, 0), (27, 1)])
+@pytest.mark.parametrize("box", [(1, 1, 1), (33, 17, 9), (31, 15, 40)])
+def test_one_component_is_lbf_step(storage, lattice, highorder, box):
+    """Without obstacles the two compilations of the one-component step give the
+    same bits.  With HIGHORDER the compiler contracts the rows in its own way in
+    each: there a step differs by the rounding of the rows, some units of 2^-24
+    (2^-53) of the result, and in 16-bit storage by values that round the other
+    way, at most half an ulp a step."""
+    p = L.Params(lx=box[0], ly=box[1], lz=box[2], lattice=lattice, highorder=highorder, smagorinsky=highorder, visc1=0.05,
+                 fx=1e-5, fy=-4e-6, storage=storage)
+    m = _random_moments(np.random.default_rng(box[0]), p.shape)
+    s = L.Solver(p)
+    s.set_fields(m)
+    s.step(6)
+    with L.Server(chunk=4) as v:
+        i = v.submit(p, m, None, 6)
+        v.drain()
+        served, alone = v.fetch(i), s.get_fields()[:2]
+    s.close()
+    if highorder:
+        assert rel_l2(served[0], alone[0]) <= {"f32": 6 * 8 * 2.0 ** -24, "f64": 6 * 8 * 2.0 ** -53, "bf16": 6 * 2.0 ** -9}[storage]
+    else:
+        assert _same(served, alone)
 
 
 def test_server_fp32_matches_oracle():
