@@ -792,8 +792,13 @@ __device__ __forceinline__ void step_body(const StepParams<S, R>& p, const int b
     }
 }
 
-// CTAs per SM the kernel is compiled for: two of 8-row tiles, one of 16 rows, one in FP64
-template <typename R, int TYV> constexpr int step_min_blocks() { return (sizeof(R) == 8 || TYV > 8) ? 1 : 2; }
+// CTAs per SM the kernel is compiled for: two of 8-row tiles, one of 16 rows, one
+// in FP64, and one of 8 rows of D3Q27 HIGHORDER with one component, whose
+// two spill up to 264 bytes in 80 registers (FP32, a step of 200^3 in 16-plane
+// segments 388 us with two, 365 us with one; of 40^3 21.3 and 13.9 us)
+template <int LAT, bool HO, bool TC, typename R, int TYV> constexpr int step_min_blocks() {
+    return (sizeof(R) == 8 || TYV > 8 || (LAT == 27 && HO && !TC)) ? 1 : 2;
+}
 
 // threads and shared memory of a CTA, by component class
 template <bool TC, int TYV> constexpr int step_threads() { return TC ? TX * TYV : single_threads<TYV>(); }
@@ -836,7 +841,7 @@ __device__ __forceinline__ void run_share(const int nx, const int nzr, const int
 // separately inlined copies may contract floating-point operations
 // differently and give results that differ in the last bit.
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
-__global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>()) stream_kernel(const StepParams<S, R> p) {
+__global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<LAT, HO, TC, R, TYV>()) stream_kernel(const StepParams<S, R> p) {
     chain_begin();
     long long s0, s1;
     const int nzr = p.zhi - p.zlo;
@@ -869,7 +874,7 @@ __global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TY
 // another compilation, where the compiler contracts the products of the
 // two-component collision differently: the two agree to rounding.
 template <int LAT, bool HO, bool TC, typename S, typename R, int TYV, bool REP = false, int OBS = 1>
-__global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<R, TYV>())
+__global__ void __launch_bounds__(step_threads<TC, TYV>(), step_min_blocks<LAT, HO, TC, R, TYV>())
     stream_kernel_batched(const StepParams<S, R>* __restrict__ boxes, const int4* __restrict__ work) {
     __shared__ StepParams<S, R> sp;
     chain_begin();
