@@ -238,10 +238,11 @@ cudaError_t launch_print(int storage, const PrintArgs& a, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------
 // FP64 sums over fluid nodes (phi_sum_count_kernel, lb_cuda_boundary_module.f90:461-515):
-// grid-stride loops on one wave of CTAs, a warp and block tree, one atomic per
-// CTA and sum.  With a CTA per 256 nodes (up to 9,472 of them) the trees and
-// atomics cost more than the loads: lbf_reduce of 256^3 (336 MB) 137 us with
-// its copy to the host, 99 us now; the phi sum of 150 x 128 x 136 35 us (ncu).
+// grid-stride loops on at most eight CTAs an SM (five or six of lbf_reduce's
+// fit at a time), a warp and block tree, one atomic per CTA and sum.  With a CTA
+// per 256 nodes (up to 9,472 of them) the trees and atomics cost more than the
+// loads: lbf_reduce with its copy to the host 131 us for 256^3 (336 MB), 81 us now;
+// 85 us for 150 x 128 x 136, 31 us now.
 // ---------------------------------------------------------------------------
 constexpr int SUM_THREADS = 256;
 static inline int sum_blocks(long long n) {
