@@ -516,6 +516,11 @@ struct IsfAt {
         }
         return isf[((long long)c[2] * n[1] + c[1]) * n[0] + c[0]];
     }
+    // a node whose neighbours need no folding
+    bool inside(int x, int y, int z) const {
+        return x > 0 && x < n[0] - 1 && y > 0 && y < n[1] - 1 && z > 0 && z < n[2] - 1;
+    }
+    long long offset(int l) const { return ((long long)EZh[l] * n[1] + EYh[l]) * n[0] + EXh[l]; }
 };
 
 // Device tables made from isfluid.  They are built apart from the handle's and
@@ -578,22 +583,21 @@ int link_tables(const lbf_handle* h, const int8_t* isf, IsfTables& t) {
     for (int l = 1; l < 27; ++l) {
         if (!link_in(lat, l)) continue;
         ls[nl++] = l;
-        up[l] = -(((long long)EZh[l] * ny + EYh[l]) * nx + EXh[l]);
+        up[l] = -isf_at.offset(l);
     }
     for (int k = 0; k < nz; ++k)
         for (int j = 0; j < ny; ++j) {
             const int8_t* row = isf + ((long long)k * ny + j) * nx;
-            const bool edge = k == 0 || k == nz - 1 || j == 0 || j == ny - 1;
             for (int x0 = 0; x0 < nx; x0 += lbf::STEP_TILE_X) {
                 rows[((size_t)k * ny + j) * segs + x0 / lbf::STEP_TILE_X] = (int)links.size();
                 const int8_t* const end = row + std::min(nx, x0 + lbf::STEP_TILE_X);
                 // the -1 nodes of the segment
                 for (const int8_t* q = row + x0; (q = static_cast<const int8_t*>(std::memchr(q, 0xff, end - q))); ++q) {
                     const int i = (int)(q - row);
-                    const bool fold = edge || i == 0 || i == nx - 1;
+                    const bool inside = isf_at.inside(i, j, k);
                     unsigned m = 0;
                     for (int n = 0; n < nl; ++n) {
-                        const int l = ls[n], f = fold ? isf_at(i - EXh[l], j - EYh[l], k - EZh[l]) : q[up[l]];
+                        const int l = ls[n], f = inside ? q[up[l]] : isf_at(i - EXh[l], j - EYh[l], k - EZh[l]);
                         m |= (unsigned)(f == 0) << l;
                     }
                     links.push_back(m);
@@ -622,6 +626,8 @@ int wet_tables(const lbf_handle* h, const int8_t* isf, IsfTables& t) {
     const int nx = h->nx, ny = h->ny, nz = h->nz, lat = h->p.lattice;
     const int dims[3] = {nx, ny, nz}, pb[3] = {h->p.pbc_x, h->p.pbc_y, h->p.pbc_z};
     const IsfAt isf_at(h, isf);
+    long long down[27];
+    for (int l = 0; l < 27; ++l) down[l] = isf_at.offset(l);
     std::vector<long long> vs;
     std::vector<int> vd, vf, vsh;
     std::vector<double> vwn;
@@ -635,11 +641,15 @@ int wet_tables(const lbf_handle* h, const int8_t* isf, IsfTables& t) {
             for (int i = 0; i < nx; ++i) {
                 long long c = ((long long)k * ny + j) * nx + i;
                 if (isf[c] != 0) continue;
+                const bool inside = isf_at.inside(i, j, k);
+                auto near = [&](int l) -> int {
+                    return inside ? isf[c + down[l]] : isf_at(i + EXh[l], j + EYh[l], k + EZh[l]);
+                };
                 double wx = 0, wy = 0, wz = 0;
                 for (int l = 1; l < 27; ++l) {
                     if (!link_in(lat, l)) continue;
                     int d2 = EXh[l] * EXh[l] + EYh[l] * EYh[l] + EZh[l] * EZh[l];
-                    if (isf_at(i + EXh[l], j + EYh[l], k + EZh[l]) == 0) continue;
+                    if (near(l) == 0) continue;
                     double sc = d2 == 1 ? 1.0 : d2 == 2 ? 0.5 : 1.0 / 3.0;
                     wx += sc * -EXh[l];
                     wy += sc * -EYh[l];
@@ -653,7 +663,7 @@ int wet_tables(const lbf_handle* h, const int8_t* isf, IsfTables& t) {
                 for (int l = 1; l < 27; ++l) {
                     if (!link_in(lat, l)) continue;
                     int d2 = EXh[l] * EXh[l] + EYh[l] * EYh[l] + EZh[l] * EZh[l];
-                    int f = isf_at(i + EXh[l], j + EYh[l], k + EZh[l]);
+                    int f = near(l);
                     if (f != 1 && f != -1) continue;
                     double sc = d2 == 1 ? 1.0 : d2 == 2 ? 0.70710678118654752440 : 0.57735026918962576450;
                     double score = (-EXh[l] * wx + -EYh[l] * wy + -EZh[l] * wz) * sc;
