@@ -15,12 +15,12 @@
 // component classes that this one replaced.
 // Bound by issue and by the latency between a plane's barriers (20 warps, 0.6
 // instructions a cycle and scheduler); registers hold it to one CTA of 16 rows
-// or two of 8 (one with HIGHORDER).  FP32, 200 x 184 x 168, a step: D3Q19 265 us in the shared body,
-// 154 us here; D3Q27 HIGHORDER with SMAGORINSKI 317 and 281 us (267 us with the
-// sums of the rows and populations regrouped, which rounds differently).
-// D3Q27 does not fit in the 96 registers of 16 rows (FP32 spills 32-36 bytes, 104-136
-// with obstacles) nor, without HIGHORDER, in the 80 of 8 rows (92 and 216 bytes);
-// FP64 spills up to 204 of its 168.
+// or two of 8 (one with HIGHORDER).  FP32, 200 x 184 x 168, a step: D3Q19 265 us
+// in the shared body, 154 us here; D3Q27 HIGHORDER with SMAGORINSKI 317 and 281 us
+// (267 us with the sums of the rows and populations regrouped, which rounds
+// differently).  D3Q27 does not fit in the 96 registers of 16 rows (FP32 spills
+// 32-36 bytes, 104-136 with obstacles) nor, without HIGHORDER, in the 80 of 8
+// rows (92 and 216 bytes); FP64, with 168, spills up to 204.
 #pragma once
 #include "lbf_node.cuh"
 
